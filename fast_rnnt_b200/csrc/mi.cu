@@ -37,7 +37,7 @@
 
 #include <mutex>
 
-#include "common.cuh"
+#include "mi.cuh"
 
 namespace frnnt {
 
@@ -49,40 +49,6 @@ constexpr int kIoWarps = 4;     // loader warps per CTA of the forward sweep
 __host__ __device__ constexpr int bwd_io_warps(int ncw) { return ncw <= 4 ? 16 : 8; }
 constexpr int kHandRing = 64;   // hand-off slots per warp (two chunks deep)
 constexpr int kSpinLimit = 1 << 22;
-
-struct MiBox {
-  int s0, t0, sb, tb;  // origin and extents (s_end - s_begin, t_end - t_begin)
-};
-
-__device__ __forceinline__ MiBox load_box(const int64_t *boundary, int b, int S, int T) {
-  MiBox box{0, 0, S, T};
-  if (boundary != nullptr) {
-    // clamped so that a malformed row can never index outside the tensors
-    int s0 = (int)boundary[4 * b + 0], t0 = (int)boundary[4 * b + 1];
-    int s1 = (int)boundary[4 * b + 2], t1 = (int)boundary[4 * b + 3];
-    s0 = max(0, min(s0, S));
-    t0 = max(0, min(t0, T));
-    s1 = max(s0, min(s1, S));
-    t1 = max(t0, min(t1, T));
-    box = MiBox{s0, t0, s1 - s0, t1 - t0};
-  }
-  return box;
-}
-
-// lattice scratch: the weight exponents by anti-diagonal, [B][S+T+1][pitch]
-__host__ __device__ inline int lattice_pitch(int S) { return (S + 1 + 31) & ~31; }
-// followed, per utterance, by two vectors of edge_elems() values: when the lattice has
-// more rows than one CTA holds it is swept in row blocks (one launch per block); the
-// forward sweep passes p of a block's last row, the backward sweep the x-gradients of
-// a block's first row, to the next launch through them
-__host__ __device__ inline size_t edge_elems(int S, int T) { return (size_t)(S + T + 1 + 2 * kChunk); }
-__host__ __device__ inline size_t lattice_elems_per_utt(int S, int T) {
-  return (size_t)(S + T + 1) * lattice_pitch(S) + 2 * edge_elems(S, T);
-}
-
-__device__ __forceinline__ void bar_sync_named(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 
 // ---- asynchronous global -> shared copies of single elements ---------------------
 // (the loader warps keep dozens of these in flight; a plain load + store loop
@@ -215,8 +181,7 @@ mi_forward_kernel(const real *__restrict__ px, const real *__restrict__ py,
   const real ninf = neg_inf<real>();
   // edge vectors behind the lattice, indexed by lattice diagonal: this block writes one
   // (p of its last row), the next block reads it
-  real *edge = lattice ? lattice + (size_t)b * lattice_elems_per_utt(S, T) + (size_t)(S + T + 1) * lpitch
-                       : nullptr;
+  real *edge = lattice ? edges_of(lattice, b, gridDim.x, S, T) : nullptr;
   const int blk = row0 / ROWS;
   real *edge_out = edge ? edge + (size_t)(blk & 1) * edge_elems(S, T) : nullptr;
   const real *edge_in = edge ? edge + (size_t)((blk + 1) & 1) * edge_elems(S, T) : nullptr;
@@ -261,9 +226,7 @@ mi_forward_kernel(const real *__restrict__ px, const real *__restrict__ py,
   real p_cur = (!MODIFIED && top_row) ? (real)0 : ninf, p_old = ninf;
   real p_last = ninf;                 // the last active value (the answer for row sb)
   typename H::slot_t early = 0;       // the neighbour's slot for the next step, read ahead
-  real *L = lattice ? lattice + (size_t)b * lattice_elems_per_utt(S, T) + (size_t)row0 * lpitch +
-                          row0 + i
-                    : nullptr;
+  real *L = lattice ? lattice_of(lattice, b, S, T) + (size_t)row0 * lpitch + row0 + i : nullptr;
 
   for (int c = 0; c < nchunks; ++c) {
     if (is_io) {
@@ -383,9 +346,9 @@ mi_backward_kernel(const real *__restrict__ px, real *__restrict__ lattice,
   real *GX = px_grad + (size_t)b * S * T1;
   real *GY = py_grad + (size_t)b * (S + 1) * T;
   const int lpitch = lattice_pitch(S);
-  const real *LT = lattice + (size_t)b * lattice_elems_per_utt(S, T);
+  const real *LT = lattice_of(lattice, b, S, T);
   // edge vectors, indexed by lattice diagonal: this block writes one, reads the other
-  real *edge = lattice + (size_t)b * lattice_elems_per_utt(S, T) + (size_t)(S + T + 1) * lpitch;
+  real *edge = edges_of(lattice, b, gridDim.x, S, T);
   const int blk = row0 / ROWS;
   real *edge_out = edge + (size_t)(blk & 1) * edge_elems(S, T);
   const real *edge_in = edge + (size_t)((blk + 1) & 1) * edge_elems(S, T);
@@ -580,219 +543,35 @@ mi_backward_kernel(const real *__restrict__ px, real *__restrict__ lattice,
   }
 }
 
-// -----------------------------------------------------------------------------
-// Backward sweep with four rows per thread (float, lattices of 33 .. 128 rows)
-// -----------------------------------------------------------------------------
-// The same reverse sweep with ONE compute warp: lane l owns lattice rows 4l .. 4l+3.  A
-// step then advances four cells per thread -- independent of each other, so their
-// multiply-add chains overlap in the pipeline -- and the only neighbour value that has to
-// travel is the one between a thread's outer rows, one warp shuffle per step.  No value
-// crosses a warp boundary, so the tagged shared-memory hand-off of the row-per-thread
-// kernel (a third of its step time) is gone: 88 -> 68 us on a 64 x (100, 500) batch.  The
-// arithmetic per cell is unchanged, so results are bit-identical to that kernel.  (The
-// forward sweep does not profit: a LogAdd is ~100 instructions, so four per thread make one
-// warp issue-bound at ~750 cycles per step against ~370 for the row-per-thread kernel:
-// 0.24 ms instead of 0.12 ms, measured; its variant was dropped.)
-constexpr int kRpt = 4;
-constexpr int kRptRows = 32 * kRpt;
-constexpr int kRptBatch = 4;  // steps whose weights are fetched together
-
-template <bool MODIFIED>
-__global__ void __launch_bounds__((1 + bwd_io_warps(kRpt)) * 32)
-mi_backward_rpt_kernel(float *__restrict__ lattice, const int64_t *__restrict__ boundary,
-                       const float *__restrict__ ans_grad, float *__restrict__ px_grad,
-                       float *__restrict__ py_grad, float *__restrict__ origin_grad, int S, int T) {
-  constexpr int ROWS = kRptRows;
-  constexpr int NIO = bwd_io_warps(kRpt);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float *ringd = reinterpret_cast<float *>(smem_raw);  // [2][ROWS][kPitch]  d1
-  float *ringx = ringd + 2 * ROWS * kPitch;            // [2][ROWS][kPitch]  d2, then d/dpx
-  float *ringy = ringx + 2 * ROWS * kPitch;            // [2][ROWS][kPitch]  d/dpy
-
-  const int b = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int T1 = MODIFIED ? T : T + 1;
-  constexpr int off = MODIFIED ? -1 : 0;
-  constexpr int tp_min_x = MODIFIED ? 1 : 0;
-  const MiBox box = load_box(boundary, b, S, T);
-  const int ib = min(ROWS - 1, box.sb);
-  const int nd = ib + box.tb + 1;
-  const int nchunks = (nd + kChunk - 1) / kChunk;
-  float *GX = px_grad + (size_t)b * S * T1;
-  float *GY = py_grad + (size_t)b * (S + 1) * T;
-  const int lpitch = lattice_pitch(S);
-  const float *LT = lattice + (size_t)b * lattice_elems_per_utt(S, T);
-  const bool is_io = warp >= 1;
-
-  // helper warps: weights of chunk c (lane = row within a block of 32, diagonals by warp)
-  auto weights_chunk = [&](int c) {
-    const int slot = c & 1;
-    const int iw = warp - 1;
-    constexpr int NJ = kChunk / NIO;
-    constexpr int NM = kRpt;
-    float dl[NJ][NM];
-#pragma unroll
-    for (int jj = 0; jj < NJ; ++jj) {
-      const int k = c * kChunk + iw + jj * NIO;
-#pragma unroll
-      for (int m = 0; m < NM; ++m) {
-        const int i = lane + 32 * m;
-        const int tp = k - i;
-        const bool v = i >= 1 && i <= ib && tp >= 1 && tp <= box.tb;
-        dl[jj][m] = v ? LT[(size_t)k * lpitch + i] : 0.f;
-      }
-    }
-    bar_sync_named(2, NIO * 32);
-#pragma unroll
-    for (int jj = 0; jj < NJ; ++jj) {
-      const int j = iw + jj * NIO;
-      const int k = c * kChunk + j;
-#pragma unroll
-      for (int m = 0; m < NM; ++m) {
-        const int i = lane + 32 * m;
-        if (i > ib) continue;
-        const int tp = k - i;
-        float d1 = 0, d2 = 0;
-        if (tp >= 0 && tp <= box.tb) {
-          if (i == 0) {
-            d2 = 1;
-          } else if (tp == 0) {
-            d1 = MODIFIED ? 0 : 1;
-          } else {
-            const float w = exp_r(dl[jj][m]);
-            if (w - w == 0) {
-              d1 = w;
-              d2 = 1.f - w;
-            }
-          }
-        }
-        ringd[(slot * ROWS + i) * kPitch + j] = d1;
-        ringx[(slot * ROWS + i) * kPitch + j] = d2;
-      }
-    }
-  };
-
-  auto drain_chunk = [&](int c) {
-    const int slot = c & 1;
-    const int k = c * kChunk + lane;
-#pragma unroll 4
-    for (int i = warp - 1; i <= ib; i += NIO) {
-      const int tp = k - i;
-      if (tp <= box.tb) {
-        if (i >= 1 && tp >= tp_min_x)
-          GX[(size_t)(box.s0 + i - 1) * T1 + (box.t0 + tp + off)] = ringx[(slot * ROWS + i) * kPitch + lane];
-        if (tp >= 1) GY[(size_t)(box.s0 + i) * T + box.t0 + tp - 1] = ringy[(slot * ROWS + i) * kPitch + lane];
-      }
-    }
-  };
-
-  if (is_io && nchunks > 0) weights_chunk(nchunks - 1);
-  __syncthreads();
-
-  if (is_io) {
-    // exact zeros outside the boundary box (mutual_information_cpu.cu:161-166)
-    const int lw = warp - 1;
-    const int cx_lo = box.t0, cx_hi = box.t0 + box.tb + off;
-    for (int r = lw; r < S; r += NIO) {
-      const bool in_rows = r >= box.s0 && r < box.s0 + box.sb;
-      for (int col = lane; col < T1; col += 32)
-        if (!in_rows || col < cx_lo || col > cx_hi) GX[(size_t)r * T1 + col] = 0;
-    }
-    const int cy_lo = box.t0, cy_hi = box.t0 + box.tb - 1;
-    for (int r = lw; r <= S; r += NIO) {
-      const bool in_rows = r >= box.s0 && r <= box.s0 + box.sb;
-      for (int col = lane; col < T; col += 32)
-        if (!in_rows || col < cy_lo || col > cy_hi) GY[(size_t)r * T + col] = 0;
-    }
-  }
-
-  const int i0 = lane * kRpt;
-  float g1_cur[kRpt], g1_old[kRpt], g2_cur[kRpt];
-  int k_inject[kRpt];
-#pragma unroll
-  for (int j = 0; j < kRpt; ++j) {
-    g1_cur[j] = g1_old[j] = g2_cur[j] = 0.f;
-    k_inject[j] = i0 + j == box.sb ? i0 + j + box.tb : -1;
-  }
-  float g_last = 0;  // gradient of row 0's last cell: what reaches the origin
-  const float g_end = ans_grad[b];
-
-  for (int c = nchunks - 1; c >= 0; --c) {
-    if (is_io) {
-      if (c + 1 < nchunks) drain_chunk(c + 1);
-      if (c >= 1) weights_chunk(c - 1);
-    } else {
-#pragma unroll 1
-      for (int j0 = kChunk - kRptBatch; j0 >= 0; j0 -= kRptBatch) {
-        float d1v[kRpt][kRptBatch], d2v[kRpt][kRptBatch];
-#pragma unroll
-        for (int j = 0; j < kRpt; ++j) {
-          const bool row_ok = i0 + j <= ib;
-          const float *rd = ringd + ((c & 1) * ROWS + i0 + j) * kPitch + j0;
-          const float *rx = ringx + ((c & 1) * ROWS + i0 + j) * kPitch + j0;
-#pragma unroll
-          for (int u = 0; u < kRptBatch; ++u) {
-            d1v[j][u] = row_ok ? rd[u] : 0.f;
-            d2v[j][u] = row_ok ? rx[u] : 0.f;
-          }
-        }
-#pragma unroll
-        for (int u = kRptBatch - 1; u >= 0; --u) {
-          const int k = c * kChunk + j0 + u;
-          float hist[kRpt];
-#pragma unroll
-          for (int j = 0; j < kRpt; ++j) hist[j] = MODIFIED ? g1_old[j] : g1_cur[j];
-          float from_below = __shfl_down_sync(0xffffffffu, hist[0], 1);
-          if (lane == 31) from_below = 0.f;
-          float n1[kRpt], n2[kRpt];
-#pragma unroll
-          for (int j = 0; j < kRpt; ++j) {
-            const float below = j == kRpt - 1 ? from_below : hist[j + 1];
-            float g = below + g2_cur[j];
-            if (k == k_inject[j]) g = g_end;
-            n1[j] = d1v[j][u] * g;
-            n2[j] = d2v[j][u] * g;
-            if (j == 0 && lane == 0) g_last = g;
-          }
-#pragma unroll
-          for (int j = 0; j < kRpt; ++j) {
-            ringx[((c & 1) * ROWS + i0 + j) * kPitch + j0 + u] = n1[j];
-            ringy[((c & 1) * ROWS + i0 + j) * kPitch + j0 + u] = n2[j];
-            g1_old[j] = g1_cur[j];
-            g1_cur[j] = n1[j];
-            g2_cur[j] = n2[j];
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (!is_io && lane == 0 && origin_grad != nullptr) origin_grad[b] = g_last;
-  if (is_io && nchunks > 0) drain_chunk(0);
-}
-
 // p in the reference's [B][S+1][T+1] layout -> the weight exponents
-// p[s-1][t+o] + px[s-1][t+o] - p[s][t] in the diagonal-major scratch
+// p[s-1][t+o] + px[s-1][t+o] - p[s][t] in the diagonal-major scratch, or (as_weights) the weights
+// themselves as the sweeps of mi_f32.cu keep them
 template <typename real>
 __global__ void mi_lattice_from_p_kernel(const real *__restrict__ p, const real *__restrict__ px,
                                          const int64_t *__restrict__ boundary,
-                                         real *__restrict__ lattice, int S, int T, int modified) {
+                                         real *__restrict__ lattice, int S, int T, int modified,
+                                         int as_weights) {
   const int b = blockIdx.y;
   const MiBox box = load_box(boundary, b, S, T);
   const int T1 = modified ? T : T + 1, off = modified ? -1 : 0;
   const real *P = p + (size_t)b * (S + 1) * (T + 1);
   const real *X = px + (size_t)b * S * T1;
   const int lpitch = lattice_pitch(S);
-  real *LT = lattice + (size_t)b * lattice_elems_per_utt(S, T);
+  real *LT = lattice_of(lattice, b, S, T);
   const int ncell = (box.sb + 1) * (box.tb + 1);
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < ncell;
        idx += gridDim.x * blockDim.x) {
     const int i = idx / (box.tb + 1), tp = idx % (box.tb + 1);
     real d = 0;  // first row / first column: the weights are fixed by position
+    if (as_weights && i >= 1 && tp == 0) d = modified ? kMiDead : 1;
     if (i >= 1 && tp >= 1) {
       const size_t up = (size_t)(box.s0 + i - 1);
       d = P[up * (T + 1) + box.t0 + tp + off] + X[up * T1 + box.t0 + tp + off] -
           P[(size_t)(box.s0 + i) * (T + 1) + box.t0 + tp];
+      if (as_weights) {
+        d = exp_r(d);
+        if (!(d - d == 0)) d = kMiDead;
+      }
     }
     LT[(size_t)(i + tp) * lpitch + i] = d;
   }
@@ -887,24 +666,11 @@ static int launch_backward_blocked(const void *px, void *lattice, const int64_t 
   return FRNNT_OK;
 }
 
-// float lattices of 33 .. 128 rows: the four-rows-per-thread reverse sweep
-template <bool MODIFIED>
-static int launch_backward_rpt(const void *px, void *lattice, const int64_t *boundary, const void *ans_grad,
-                               void *px_grad, void *py_grad, void *origin_grad, int B, int S, int T,
-                               cudaStream_t st) {
-  (void)px;
-  auto kern = mi_backward_rpt_kernel<MODIFIED>;
-  const size_t smem = (size_t)(3 * 2 * kRptRows) * kPitch * sizeof(float);
-  FRNNT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  FRNNT_KERNEL(kern<<<B, (1 + bwd_io_warps(kRpt)) * 32, smem, st>>>((float *)lattice, boundary,
-                                                                   (const float *)ans_grad, (float *)px_grad,
-                                                                   (float *)py_grad, (float *)origin_grad, S, T));
-  FRNNT_CUDA(cudaGetLastError());
-  return FRNNT_OK;
-}
-
-static bool mi_use_rpt(int dtype, int ncw) {
-  if (dtype != FRNNT_F32 || ncw < 2 || ncw > kRpt) return false;
+// The float sweeps are those of mi_f32.cu.  The row-per-thread kernels of this file serve
+// double, a lattice scratch that is not 16-byte aligned (the others move four values at
+// once) and FRNNT_MI=row_per_thread.
+static bool mi_use_f32(int dtype, const void *lattice) {
+  if (dtype != FRNNT_F32 || (uintptr_t)lattice % 16 != 0) return false;
   const char *mode = getenv("FRNNT_MI");
   return !(mode != nullptr && strcmp(mode, "row_per_thread") == 0);
 }
@@ -1011,6 +777,9 @@ extern "C" int frnnt_mi_forward(int dtype, const void *px, const void *py,
                 "the lattice scratch",
                 S + 1);
   cudaStream_t st = (cudaStream_t)stream;
+  if (mi_use_f32(dtype, lattice))
+    return launch_mi_forward_f32((const float *)px, (const float *)py, boundary, (float *)p, (float *)ans,
+                                 (float *)lattice, B, S, T, modified, st);
   MI_DISPATCH(launch_forward, dtype, modified, ncw, px, py, boundary, p, ans, lattice, B, S, T, st);
   return FRNNT_OK;
 }
@@ -1029,11 +798,9 @@ extern "C" int frnnt_mi_backward_from_lattice(int dtype, const void *px, void *l
                     (py_grad != nullptr || T == 0),
                 FRNNT_EINVAL, "px_grad or py_grad is NULL");
   cudaStream_t st = (cudaStream_t)stream;
-  if (mi_use_rpt(dtype, ncw))
-    return modified ? launch_backward_rpt<true>(px, lattice, boundary, ans_grad, px_grad, py_grad, origin_grad,
-                                                B, S, T, st)
-                    : launch_backward_rpt<false>(px, lattice, boundary, ans_grad, px_grad, py_grad, origin_grad,
-                                                 B, S, T, st);
+  if (mi_use_f32(dtype, lattice))
+    return launch_mi_backward_f32((float *)lattice, boundary, (const float *)ans_grad, (float *)px_grad,
+                                  (float *)py_grad, (float *)origin_grad, B, S, T, modified, st);
   MI_DISPATCH(launch_backward, dtype, modified, ncw, px, lattice, boundary, ans_grad, px_grad,
               py_grad, origin_grad, B, S, T, st);
   return FRNNT_OK;
@@ -1054,10 +821,11 @@ extern "C" int frnnt_mi_backward(int dtype, const void *px, const void *py,
   dim3 grid((unsigned)min(64, ((S + 1) * (T + 1) + 255) / 256), (unsigned)B);
   if (dtype == FRNNT_F32)
     FRNNT_KERNEL(mi_lattice_from_p_kernel<float><<<grid, 256, 0, st>>>(
-        (const float *)p, (const float *)px, boundary, (float *)lattice, S, T, modified));
+        (const float *)p, (const float *)px, boundary, (float *)lattice, S, T, modified,
+        mi_use_f32(dtype, lattice)));
   else
     FRNNT_KERNEL(mi_lattice_from_p_kernel<double><<<grid, 256, 0, st>>>(
-        (const double *)p, (const double *)px, boundary, (double *)lattice, S, T, modified));
+        (const double *)p, (const double *)px, boundary, (double *)lattice, S, T, modified, 0));
   FRNNT_CUDA(cudaGetLastError());
   return frnnt_mi_backward_from_lattice(dtype, px, lattice, boundary, ans_grad, px_grad, py_grad,
                                         origin_grad, B, S, T, modified, stream);
