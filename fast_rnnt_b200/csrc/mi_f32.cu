@@ -9,17 +9,20 @@
 //     per lane and step travels between threads (a warp shuffle).  R = 1 up to 32 rows, else
 //     2: the second row's instructions fit into the latency of the first row's chain, a third
 //     and fourth would not;
-//   * a taller lattice is split over a cluster of up to 8 CTAs.  CTA w works one chunk of 16
-//     diagonals behind CTA w - 1 (forward; the other way round in the backward): its neighbour
-//     stores the values of the edge row straight into its shared memory, and the cluster
-//     barrier that ends every chunk publishes them, so nothing is polled for.  Several
-//     compute warps on one SM were measured slower: they and their helpers share its
-//     schedulers;
+//   * a taller lattice is split over a cluster of up to 8 CTAs.  CTA w works two chunks of 16
+//     diagonals behind CTA w - 1 (forward; the other way round in the backward): the compute
+//     warp leaves the edge row in shared memory, an otherwise idle warp sends it, a chunk at
+//     a time, to the neighbour (st.async, counted by an mbarrier per chunk); an mbarrier in
+//     the other direction bounds how far the sender runs ahead.  Measured slower, in cycles a
+//     step: the compute warp sending each value itself + 55; a cluster barrier or a release at
+//     cluster scope per chunk, which waits for the helpers' global stores, + 45 to 80;
+//     several compute warps on one SM, which share its schedulers with their helpers;
 //   * helper warps move everything between global memory and shared memory, one chunk ahead
 //     (px, py, weights) and one behind (weights, gradients).  The rings are [16
 //     diagonals][rows], so that a compute lane fetches or leaves its R rows in one access;
 //     the pitch (rows + 4) keeps the transposing accesses of the helpers free of bank
-//     conflicts.  The warp that would share the compute warp's scheduler stays idle;
+//     conflicts.  The warp that shares the compute warp's scheduler is the one that only
+//     sends the edge row;
 //   * cells outside the box need no test in the forward chain: they are fed x = -inf, y = 0,
 //     which keeps rows that have not begun at -inf and the origin at 0;
 //   * LogAdd is hi + log1p(e), e = exp(-|a - b|), both written out for the range that occurs
@@ -36,9 +39,9 @@
 namespace frnnt {
 
 constexpr int kStep = 16;      // anti-diagonals per chunk
-constexpr int kHelpers = 6;    // helper warps: 1, 2, 3, 5, 6, 7 of eight (0 computes, 4 idles)
+constexpr int kHelpers = 6;    // helper warps: 1, 2, 3, 5, 6, 7 of eight (0 computes)
 constexpr int kThreads = 256;
-constexpr int kEdgeRing = 64;  // edge-row values kept (four chunks)
+constexpr int kEdgeRing = 128;  // edge-row values kept (eight chunks)
 constexpr int kMaxCluster = 8;
 
 // (log1p(e) - e) / e^2 on [0, 1] as a polynomial in e - 1/2 (minimax fit by Lawson iteration,
@@ -98,23 +101,59 @@ __device__ __forceinline__ int cluster_size() {
   return (int)r;
 }
 // address of `p` (own shared memory) in the shared memory of CTA `rank` of the cluster
-__device__ __forceinline__ unsigned peer_address(const float *p, int rank) {
+__device__ __forceinline__ unsigned peer_address(const void *p, int rank) {
   unsigned a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
                : "=r"(a)
                : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
   return a;
 }
-__device__ __forceinline__ void peer_store(unsigned address, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory");
+// `v` to an address in a peer's shared memory; counts four bytes at that CTA's mbarrier `bar`
+__device__ __forceinline__ void peer_send(unsigned address, float v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(address),
+               "r"(__float_as_uint(v)), "r"(bar)
+               : "memory");
 }
-template <bool CLUSTER>
-__device__ __forceinline__ void chunk_barrier() {
-  if (CLUSTER)
-    cooperative_groups::this_cluster().sync();
-  else
-    __syncthreads();
+
+// Hand-over of the edge row between neighbouring CTAs, chunks numbered in the order of the sweep.
+// Each side has one mbarrier per slot of the edge ring (chunk mod 4): `full` in the consumer's
+// shared memory, `taken` in the producer's.  Every wait is bounded; one that runs out makes
+// all later ones give up at once (and the caller's results NaN).
+constexpr int kSlots = kEdgeRing / kStep;
+constexpr int kSpinLimit = 1 << 22;
+
+__device__ __forceinline__ void slot_init(uint64_t *bars) {
+  for (int i = 0; i < 2 * kSlots; ++i)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(bars + i)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+// "taken" carries no data: what it lets the producer overwrite has been read into registers
+__device__ __forceinline__ void slot_arrive(unsigned peer_bars, int chunk) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(peer_bars + 8 * (chunk % kSlots)) : "memory");
+}
+// the receiver's own arrival: `steps` values are to come for this chunk
+__device__ __forceinline__ void slot_expect(uint64_t *bars, int chunk, int steps) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(bars + chunk % kSlots)),
+               "r"(4 * steps)
+               : "memory");
+}
+__device__ __forceinline__ bool slot_wait(const uint64_t *bars, int chunk, bool failed) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(bars + chunk % kSlots);
+  const unsigned parity = (chunk / kSlots) & 1;
+  for (int spin = 0; !failed; ++spin) {
+    unsigned done;
+    asm volatile("{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n"
+                 "selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(done)
+                 : "r"(a), "r"(parity)
+                 : "memory");
+    if (done) return false;
+    failed = spin >= kSpinLimit;
+  }
+  return true;
+}
+__device__ __forceinline__ void cluster_sync() { cooperative_groups::this_cluster().sync(); }
 
 template <int R>
 struct MiShape {
@@ -125,7 +164,7 @@ struct MiShape {
   static constexpr int kQuads = kRows / 4 * kStep;            // of weights in a chunk, four rows each
   static constexpr int kQuadsPerLane = (kQuads + kHelpers * 32 - 1) / (kHelpers * 32);
   static constexpr int kGroup = 8;                            // steps whose inputs are fetched together
-  static constexpr size_t kSmem = ((size_t)6 * kStep * kRing + kEdgeRing) * sizeof(float);
+  static constexpr size_t kSmem = ((size_t)6 * kStep * kRing + kEdgeRing + 2 * kStep) * sizeof(float) + 2 * kSlots * sizeof(uint64_t);
 };
 
 // -----------------------------------------------------------------------------
@@ -146,6 +185,9 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
   float *ringw = ringy + 2 * kStep * PITCH;      // [2][kStep][PITCH]  exponents of the weights
   // p by block diagonal (mod kEdgeRing) of the row above this CTA's first row
   float *above = ringw + 2 * kStep * PITCH;
+  // [kSlots] edge row arrived from the CTA above, [kSlots] edge row taken by the CTA below
+  uint64_t *bars = reinterpret_cast<uint64_t *>(above + kEdgeRing);
+  float *own = reinterpret_cast<float *>(bars + 2 * kSlots);  // [2][kStep]  p of this CTA's last row
   const int rank = CLUSTER ? cluster_rank() : 0, ranks = CLUSTER ? cluster_size() : 1;
   const int row0 = BLOCKED ? row0_arg : 0;
   const int b = blockIdx.x / ranks;
@@ -159,7 +201,6 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
   const int first = rank * ROWS;
   const int nd = ib + box.tb + 1;
   const int nchunks = (nd + kStep - 1) / kStep;
-  const int niter = nchunks + ib / ROWS;         // the last CTA with rows is that many chunks behind
   const float *X = px + (size_t)b * S * T1;
   const float *Y = py + (size_t)b * (S + 1) * T;
   const int lpitch = lattice_pitch(S);
@@ -171,21 +212,29 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
   const bool keep = lattice != nullptr;
   const bool has_rows = first <= ib;
 
-  if (threadIdx.x < kEdgeRing) above[threadIdx.x] = ninf;
+  for (int j = threadIdx.x; j < kEdgeRing; j += kThreads) above[j] = ninf;
+  if (CLUSTER) {
+    if (threadIdx.x == 0) slot_init(bars);
+    cluster_sync();
+    if (!has_rows) {
+      cluster_sync();  // the one at the end
+      return;
+    }
+  }
 
   // Helper warps.  A lane takes R rows of one diagonal at a time: fetch() reads
   // x = px[s0+i-1][t0+t'+o] and y = py[s0+i][t0+t'-1] of the cells (row i, diagonal k) of
-  // iteration `it` into registers, place() stores them in the rings one barrier later, so
+  // chunk c into registers, place() stores them in the rings one barrier later, so
   // that a whole chunk's time covers the latency of global memory.
   const bool helper = (warp & 3) != 0;
   const int hw = warp - 1 - (warp >> 2), hj = lane & (kStep - 1), half = lane / kStep;
   float xv[M::kTasksPerWarp][R], yv[M::kTasksPerWarp][R], ev = ninf;
-  auto fetch = [&](int it) {
+  auto fetch = [&](int c) {
 #pragma unroll
     for (int n = 0; n < M::kTasksPerWarp; ++n) {
       const int task = hw + n * kHelpers;
       const int q0 = first + R * (2 * task + half);
-      const int tp0 = (it - rank) * kStep + hj - q0;  // t' of the first row's cell
+      const int tp0 = c * kStep + hj - q0;  // t' of the first row's cell
       const float *xs = X + (long long)(box.s0 + row0 + q0 - 1) * T1 + (box.t0 + tp0 + off);
       const float *ys = Y + (long long)(box.s0 + row0 + q0) * T + (box.t0 + tp0 - 1);
 #pragma unroll
@@ -199,35 +248,35 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
     }
     if (BLOCKED && rank == 0 && row0 > 0 && hw == 0 && lane < kStep) {
       // p of cell (row0 - 1, t') of the block above; the steps of a chunk read diagonals up to
-      // kStep * it + kStep - 2
-      const int d = it * kStep - 1 + lane;
+      // kStep * c + kStep - 2
+      const int d = c * kStep - 1 + lane;
       ev = d + 1 <= box.tb ? edge_in[row0 + d] : ninf;
     }
   };
-  auto place = [&](int it) {
+  auto place = [&](int c) {
 #pragma unroll
     for (int n = 0; n < M::kTasksPerWarp; ++n) {
       const int task = hw + n * kHelpers;
-      const int at = ((it & 1) * kStep + hj) * PITCH + R * (2 * task + half);
+      const int at = ((c & 1) * kStep + hj) * PITCH + R * (2 * task + half);
       if (task < M::kTasks) {
         store_rows<R>(ringx + at, xv[n]);
         store_rows<R>(ringy + at, yv[n]);
       }
     }
     if (BLOCKED && rank == 0 && row0 > 0 && hw == 0 && lane < kStep)
-      above[(it * kStep - 1 + lane + kEdgeRing) % kEdgeRing] = ev;
+      above[(c * kStep - 1 + lane + kEdgeRing) % kEdgeRing] = ev;
   };
-  // weights of what iteration `it` left in ringw, four rows of one diagonal at a time
+  // weights of what chunk c left in ringw, four rows of one diagonal at a time
   float *L = keep ? lattice_of(lattice, b, S, T) + (size_t)row0 * lpitch + row0 : nullptr;
-  auto weights = [&](int it) {
+  auto weights = [&](int c) {
 #pragma unroll
     for (int n = 0; n < M::kQuadsPerLane; ++n) {
       const int q = (n * kHelpers + hw) * 32 + lane;
       const int l0 = 4 * (q % (ROWS / 4)), j = q / (ROWS / 4), q0 = first + l0;
-      const int k = (it - rank) * kStep + j;
+      const int k = c * kStep + j;
       if (q >= M::kQuads || k < 0 || k >= nd || row0 + q0 >= lpitch) continue;
       float w[4];
-      load_rows<4>(w, ringw + ((it & 1) * kStep + j) * PITCH + l0);
+      load_rows<4>(w, ringw + ((c & 1) * kStep + j) * PITCH + l0);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         w[r] = expf(w[r]);
@@ -240,12 +289,12 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
   };
 
   if (BLOCKED) __syncthreads();  // `above` is filled by the helpers, too
-  if (helper && has_rows) {
+  if (helper) {
     fetch(0);
     place(0);
-    if (niter > 1) fetch(1);
+    if (nchunks > 1) fetch(1);
   }
-  chunk_barrier<CLUSTER>();
+  __syncthreads();
 
   const int i0 = first + lane * R;               // this lane's first block row
   float p_cur[R], p_old[R];
@@ -256,22 +305,35 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
     p_old[r] = ninf;
   }
   float *P = WRITE_P ? p + (size_t)b * (S + 1) * (T + 1) : nullptr;
-  // the last lane hands its last row to the next CTA
-  const bool hand_down = CLUSTER && lane == 31 && rank + 1 < ranks;
-  const unsigned next = hand_down ? peer_address(above, rank + 1) : 0u;
+  // this CTA's last row for the one below, by the warp that has nothing else to do
+  const bool has_next = CLUSTER && first + ROWS <= ib;
+  const bool sender = CLUSTER && warp == 4;
+  const unsigned next = has_next ? peer_address(above, rank + 1) : 0u;
+  const unsigned next_full = has_next ? peer_address(bars, rank + 1) : 0u;
+  const unsigned prev_taken = CLUSTER && rank > 0 ? peer_address(bars + kSlots, rank - 1) : 0u;
+  auto pass_on = [&](int c) {
+    if (rank > 0 && lane == 0) slot_arrive(prev_taken, c);
+    if (has_next && lane < min(kStep, nd - c * kStep)) {
+      const bool late = c >= kSlots - 1 && slot_wait(bars + kSlots, c - (kSlots - 1), false);
+      peer_send(next + 4 * ((c * kStep + lane) & (kEdgeRing - 1)), late ? NAN : own[(c & 1) * kStep + lane],
+                next_full + 8 * (c % kSlots));
+    }
+  };
+  bool failed = false;
 
-  for (int it = 0; it < niter; ++it) {
-    const int c = it - rank;
-    if (!has_rows) {
-      // only the barriers
-    } else if (helper) {
-      if (it + 1 < niter) place(it + 1);
-      if (it + 2 < niter) fetch(it + 2);
-      if (keep && it >= 1) weights(it - 1);
-    } else if (warp == 0 && c >= 0 && c < nchunks) {
-      float *rw = ringw + (it & 1) * kStep * PITCH + lane * R;
-      const float *rx = ringx + (it & 1) * kStep * PITCH + lane * R;
-      const float *ry = ringy + (it & 1) * kStep * PITCH + lane * R;
+  for (int c = 0; c < nchunks; ++c) {
+    if (helper) {
+      if (c + 1 < nchunks) place(c + 1);
+      if (c + 2 < nchunks) fetch(c + 2);
+      if (keep && c >= 1) weights(c - 1);
+    } else if (warp == 0) {
+      if (CLUSTER && rank > 0) {
+        if (lane == 0) slot_expect(bars, c, min(kStep, nd - c * kStep));
+        failed = slot_wait(bars, c, failed);
+      }
+      float *rw = ringw + (c & 1) * kStep * PITCH + lane * R;
+      const float *rx = ringx + (c & 1) * kStep * PITCH + lane * R;
+      const float *ry = ringy + (c & 1) * kStep * PITCH + lane * R;
       const int nstep = min(kStep, nd - c * kStep);
       float x[2][G][R], y[2][G][R], nb[2][G];
       auto inputs = [&](int j0, int s) {
@@ -303,7 +365,7 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
           p_old[r] = p_cur[r];
           p_cur[r] = pn[r];
         }
-        if (hand_down) peer_store(next + 4 * (k & (kEdgeRing - 1)), p_cur[R - 1]);
+        if (CLUSTER && lane == 31) own[(c & 1) * kStep + j] = p_cur[R - 1];
         if (keep) store_rows<R>(rw + j * PITCH, dl);
         if (BLOCKED && i0 + R == kMiF32Rows) edge_out[row0 + k] = p_cur[R - 1];
         if (WRITE_P) {
@@ -333,16 +395,20 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
             if (j0 + u < nstep) step(j0 + u, x[0][u], y[0][u], nb[0][u]);
         }
       }
+    } else if (sender && c >= 1) {
+      pass_on(c - 1);
     }
-    chunk_barrier<CLUSTER>();
+    __syncthreads();
   }
-  if (helper && has_rows && keep) weights(niter - 1);
+  if (helper && keep) weights(nchunks - 1);
+  if (sender) pass_on(nchunks - 1);
   // the last step of a row is diagonal nd - 1, where the last row reaches its end
   if (warp == 0) {
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (row0 + i0 + r == box.sb) ans[b] = p_cur[r];
+      if (row0 + i0 + r == box.sb) ans[b] = failed ? NAN : p_cur[r];
   }
+  if (CLUSTER) cluster_sync();  // the neighbours may still be writing here
 }
 
 // -----------------------------------------------------------------------------
@@ -363,6 +429,9 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
   float *ringw = ringy + 2 * kStep * PITCH;      // [2][kStep][PITCH]  weights
   // x-gradients by block diagonal (mod kEdgeRing) of the row below this CTA's last row
   float *below = ringw + 2 * kStep * PITCH;
+  // [kSlots] edge row arrived from the CTA below, [kSlots] edge row taken by the CTA above
+  uint64_t *bars = reinterpret_cast<uint64_t *>(below + kEdgeRing);
+  float *own = reinterpret_cast<float *>(bars + 2 * kSlots);  // [2][kStep]  this CTA's first row
   const int rank = CLUSTER ? cluster_rank() : 0, ranks = CLUSTER ? cluster_size() : 1;
   const int row0 = BLOCKED ? row0_arg : 0;
   const int b = blockIdx.x / ranks;
@@ -373,8 +442,6 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
   const int first = rank * ROWS;
   const int nd = ib >= 0 ? ib + box.tb + 1 : 0;
   const int nchunks = (nd + kStep - 1) / kStep;
-  const int last_rank = ib >= 0 ? ib / ROWS : 0;  // it leads
-  const int niter = nd > 0 ? nchunks + last_rank : 0;
   float *GX = px_grad + (size_t)b * S * T1;
   float *GY = py_grad + (size_t)b * (S + 1) * T;
   const int lpitch = lattice_pitch(S);
@@ -386,15 +453,15 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
   const bool block_below = BLOCKED && row0 + kMiF32Rows <= box.sb;
   const bool has_rows = first <= ib;
 
-  if (threadIdx.x < kEdgeRing) below[threadIdx.x] = 0.f;
+  for (int j = threadIdx.x; j < kEdgeRing; j += kThreads) below[j] = 0.f;
   if (BLOCKED) __syncthreads();  // `below` is filled by the helpers, too
 
-  // chunk that this CTA works on at iteration `it`
-  auto chunk_of = [&](int it) { return nchunks - 1 - (it - (last_rank - rank)); };
+  // the chunk of diagonals that is the n-th of the sweep
+  auto chunk_of = [&](int n) { return nchunks - 1 - n; };
 
-  // Helper warps.  fetch() reads the weights of iteration `it` into registers (four rows of one
+  // Helper warps.  fetch() reads the weights of the it-th chunk into registers (four rows of one
   // diagonal per lane), place() stores them in the ring one barrier later; drain() writes the
-  // gradients of an iteration out, a lane taking R rows of one diagonal at a time.
+  // gradients of a chunk out, a lane taking R rows of one diagonal at a time.
   const bool helper = (warp & 3) != 0;
   const int hw = warp - 1 - (warp >> 2), hj = lane & (kStep - 1), half = lane / kStep;
   float wv[M::kQuadsPerLane][4], ev = 0.f;
@@ -431,7 +498,6 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
   };
   auto drain = [&](int it) {
     const int c = chunk_of(it);
-    if (c < 0 || c >= nchunks) return;
 #pragma unroll
     for (int n = 0; n < M::kTasksPerWarp; ++n) {
       const int task = hw + n * kHelpers;
@@ -454,12 +520,17 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
     }
   };
 
-  if (helper && has_rows && niter > 0) {
+  if (CLUSTER && threadIdx.x == 0) slot_init(bars);
+  const bool works = has_rows && nchunks > 0;
+  if (helper && works) {
     fetch(0);
     place(0);
-    if (niter > 1) fetch(1);
+    if (nchunks > 1) fetch(1);
   }
-  chunk_barrier<CLUSTER>();
+  if (CLUSTER)
+    cluster_sync();
+  else
+    __syncthreads();
 
   if (helper && row0 == 0) {
     // exact zeros outside the boundary box (mutual_information_cpu.cu:161-166), dealt out over
@@ -491,19 +562,34 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
     // cell (sb, tb) is its row's first step (diagonal nd - 1)
     g2_cur[r] = row0 + i0 + r == box.sb ? g_end : 0.f;
   }
-  // the first lane hands its first row's x-gradient to the CTA above
-  const bool hand_up = CLUSTER && lane == 0 && rank > 0;
-  const unsigned previous = hand_up ? peer_address(below, rank - 1) : 0u;
-
-  for (int it = 0; it < niter; ++it) {
+  // this CTA's first row for the one above, by the warp that has nothing else to do
+  const bool has_next = CLUSTER && first + ROWS <= ib;  // rows below
+  const bool sender = CLUSTER && warp == 4;
+  const unsigned previous = CLUSTER && rank > 0 ? peer_address(below, rank - 1) : 0u;
+  const unsigned previous_full = CLUSTER && rank > 0 ? peer_address(bars, rank - 1) : 0u;
+  const unsigned next_taken = has_next ? peer_address(bars + kSlots, rank + 1) : 0u;
+  auto pass_on = [&](int it) {
     const int c = chunk_of(it);
-    if (!has_rows) {
-      // only the barriers
-    } else if (helper) {
-      if (it + 1 < niter) place(it + 1);
-      if (it + 2 < niter) fetch(it + 2);
+    if (has_next && lane == 0) slot_arrive(next_taken, it);
+    if (rank > 0 && lane < min(kStep, nd - c * kStep)) {
+      const bool late = it >= kSlots - 1 && slot_wait(bars + kSlots, it - (kSlots - 1), false);
+      peer_send(previous + 4 * ((c * kStep + lane) & (kEdgeRing - 1)), late ? NAN : own[(it & 1) * kStep + lane],
+                previous_full + 8 * (it % kSlots));
+    }
+  };
+  bool failed = false;
+
+  for (int it = 0; works && it < nchunks; ++it) {
+    const int c = chunk_of(it);
+    if (helper) {
+      if (it + 1 < nchunks) place(it + 1);
+      if (it + 2 < nchunks) fetch(it + 2);
       if (it >= 1) drain(it - 1);
-    } else if (warp == 0 && c >= 0 && c < nchunks) {
+    } else if (warp == 0) {
+      if (has_next) {
+        if (lane == 0) slot_expect(bars, it, min(kStep, nd - c * kStep));
+        failed = slot_wait(bars, it, failed);
+      }
       float *rx = ringx + (it & 1) * kStep * PITCH + lane * R;
       float *ry = ringy + (it & 1) * kStep * PITCH + lane * R;
       const float *rw = ringw + (it & 1) * kStep * PITCH + lane * R;
@@ -535,7 +621,7 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
         }
         store_rows<R>(rx + j * PITCH, g1_cur);
         store_rows<R>(ry + j * PITCH, g2_cur);
-        if (hand_up) peer_store(previous + 4 * (k & (kEdgeRing - 1)), g1_cur[0]);
+        if (CLUSTER && lane == 0) own[(it & 1) * kStep + j] = g1_cur[0];
         if (BLOCKED && row0 > 0 && i0 == 0) edge_out[row0 + k] = g1_cur[0];
       };
       if (nstep == kStep) {
@@ -556,11 +642,23 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
             if (j0 + u < nstep) step(j0 + u, w[0][u], nb[0][u]);
         }
       }
+    } else if (sender && it >= 1) {
+      pass_on(it - 1);
     }
-    chunk_barrier<CLUSTER>();
+    __syncthreads();
   }
-  if (helper && has_rows && niter > 0) drain(niter - 1);
-  if (threadIdx.x == 0 && rank == 0 && row0 == 0 && origin_grad != nullptr) origin_grad[b] = g_first;
+  if (helper && works) drain(nchunks - 1);
+  if (sender && works) pass_on(nchunks - 1);
+  if (threadIdx.x == 0 && rank == 0 && row0 == 0 && origin_grad != nullptr) origin_grad[b] = failed ? NAN : g_first;
+  // a wait that ran out: say so where the caller looks (an in-box entry of this CTA's rows)
+  __syncthreads();
+  if (CLUSTER && failed && threadIdx.x == 0) {
+    if (box.tb >= 1)
+      GY[(size_t)(box.s0 + row0 + first) * T + box.t0] = NAN;
+    else if (row0 + first < box.sb)
+      GX[(size_t)(box.s0 + row0 + first) * T1 + box.t0] = NAN;
+  }
+  if (CLUSTER) cluster_sync();  // the neighbours may still be writing here
 }
 
 // -----------------------------------------------------------------------------
