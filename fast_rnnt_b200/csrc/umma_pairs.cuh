@@ -41,6 +41,11 @@
 //                                                  store_box() is called instead of finish(),
 //                                                  staging and the TMA store, for the 32-column
 //                                                  boxes of a tile from the last to the first
+//   static constexpr int kGroup;                   (optional, default kPairGroup) K slices per
+//                                                  accumulator group
+//   static constexpr bool kRowStore;               (optional, default false) boxes leave by coalesced
+//                                                  stores, a row segment each, instead of TMA: outputs
+//                                                  whose rows are not a multiple of 16 bytes
 //   struct Row;                                    per-row state across one tile's columns
 //   void row_begin(Row &, int z, int m, int n0) const;
 //   void prefetch(Row &, int z, int m, int n) const;      columns n..n+31 come next: loads
@@ -178,11 +183,30 @@ __device__ __forceinline__ PairTile pair_tile(const LinShape &p, int w) {
   return t;
 }
 
+template <class Ext, class = void>
+struct PairRowStore {
+  static constexpr bool value = false;
+};
+template <class Ext>
+struct PairRowStore<Ext, decltype((void)Ext::kRowStore)> {
+  static constexpr bool value = Ext::kRowStore;
+};
+
+template <class Ext, class = void>
+struct PairGroup {
+  static constexpr int value = kPairGroup;
+};
+template <class Ext>
+struct PairGroup<Ext, decltype((void)Ext::kGroup)> {
+  static constexpr int value = Ext::kGroup;
+};
+
 template <bool A_MN, bool B_MN, class Ext>
 __global__ void __launch_bounds__(kPairThreads, 1)
 pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
                  const __grid_constant__ CUtensorMap map_bhi, const __grid_constant__ CUtensorMap map_blo,
-                 const __grid_constant__ CUtensorMap map_out, LinShape p, Ext ext) {
+                 const __grid_constant__ CUtensorMap map_out, float *__restrict__ out, LinShape p, Ext ext) {
+  constexpr int GROUP = PairGroup<Ext>::value;
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t bar_full[kPairStages];   // TMA bytes have landed
   __shared__ __align__(8) uint64_t bar_empty[kPairStages];  // the MMAs are done with the stage
@@ -269,7 +293,7 @@ pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
         const PairTile t = pair_tile<Ext::kBatched>(p, w);
         for (int kb = 0; kb < t.KB && !*vfailed; ++kb, ++it) {
           const int s = it % kPairStages;
-          const bool group_start = kb % kPairGroup == 0;
+          const bool group_start = kb % GROUP == 0;
           // this accumulator was last used two groups ago: it must have been folded away
           if (group_start && gg >= 2 && !mbar_wait_watch(&bar_fold[gg & 1], (uint32_t)(((gg - 2) >> 1) & 1), vfailed)) {
             *vfailed = 1;
@@ -282,18 +306,19 @@ pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
           tc_fence_after_sync();
           const uint32_t acc = tmem_d + ((gg & 1) ? kPairAcc1 : 0u);
           const uint32_t st = tiles + (uint32_t)s * kPairStageBytes;
+          // the small products first: what the accumulator cuts off when it adds scales with what
+          // it holds by then
 #pragma unroll
-          for (int ks = 0; ks < kPairBK / 16; ++ks) {
-            const uint64_t dah = smem_desc_sw128(st + ks * a_step, a_lbo, 1024u);
-            const uint64_t dal = smem_desc_sw128(st + kPairOpBytes + ks * a_step, a_lbo, 1024u);
-            const uint64_t dbh = smem_desc_sw128(st + 2 * kPairOpBytes + ks * b_step, b_lbo, 1024u);
-            const uint64_t dbl = smem_desc_sw128(st + 3 * kPairOpBytes + ks * b_step, b_lbo, 1024u);
-            mma_f16_ss(acc, dah, dbh, idesc, (!group_start || ks > 0) ? 1u : 0u);
-            mma_f16_ss(acc, dah, dbl, idesc, 1u);
-            mma_f16_ss(acc, dal, dbh, idesc, 1u);
+          for (int q = 0; q < 3; ++q) {
+#pragma unroll
+            for (int ks = 0; ks < kPairBK / 16; ++ks) {
+              const uint64_t da = smem_desc_sw128(st + (q == 0 ? kPairOpBytes : 0) + ks * a_step, a_lbo, 1024u);
+              const uint64_t db = smem_desc_sw128(st + (q == 1 ? 3 : 2) * kPairOpBytes + ks * b_step, b_lbo, 1024u);
+              mma_f16_ss(acc, da, db, idesc, (!group_start || q > 0 || ks > 0) ? 1u : 0u);
+            }
           }
           mma_commit(&bar_empty[s]);
-          if (kb % kPairGroup == kPairGroup - 1 || kb == t.KB - 1) {
+          if (kb % GROUP == GROUP - 1 || kb == t.KB - 1) {
             mma_commit(&bar_grp[item & 1][gg & 1]);
             ++gg;
           }
@@ -313,7 +338,7 @@ pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
     int seen[2] = {0, 0};  // phases this set has consumed on its two barriers
     for (int w = blockIdx.x; w < n_items; w += gridDim.x, ++item) {
       const PairTile t = pair_tile<Ext::kBatched>(p, w);
-      const int NG = (t.KB + kPairGroup - 1) / kPairGroup;
+      const int NG = (t.KB + GROUP - 1) / GROUP;
       if ((item & 1) != set) {  // the other set's tile
         gg += NG;
         continue;
@@ -401,7 +426,7 @@ pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
           for (int i = 0; i < 16; ++i) v0[i] = v1[i] = NAN;
         }
         // the store of the previous box must have read the staging buffer
-        if (lane == 0) tma_store_wait_read();
+        if (!PairRowStore<Ext>::value && lane == 0) tma_store_wait_read();
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -410,9 +435,19 @@ pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
           *reinterpret_cast<float4 *>(box_ptr + sw128_offset(lane, 4 + j)) =
               make_float4(v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
         }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) tma_store_3d(&map_out, box, n, t.m0 + 32 * quarter, t.z);
+        if (PairRowStore<Ext>::value) {
+          __syncwarp();
+          // lane <-> column: 128 consecutive bytes of one row per store
+          const int m_first = t.m0 + 32 * quarter, rows = min(32, p.M - m_first);
+          float *dst = out + ((size_t)t.z * p.M + m_first) * p.N + n + lane;
+          if (n + lane < p.N)
+            for (int r = 0; r < rows; ++r, dst += p.N)
+              *dst = *reinterpret_cast<const float *>(box_ptr + sw128_offset(r, lane >> 2) + 4 * (lane & 3));
+        } else {
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) tma_store_3d(&map_out, box, n, t.m0 + 32 * quarter, t.z);
+        }
       }
       }
       if (row_ok) ext.row_end(rs, t.z, m, t.n0);
@@ -481,8 +516,15 @@ int launch_pair_umma(const CUtensorMap &mah, const CUtensorMap &mal, const CUten
                      const CUtensorMap &mbl, float *out, const LinShape &shape, const Ext &ext,
                      cudaStream_t st) {
   CUtensorMap mo;
-  // a policy that stores the result itself never uses the map, which still has to be valid
-  int rc = Ext::kCustomStore ? make_out_map(&mo, out, 1, 4, 4) : make_out_map(&mo, out, shape.nz, shape.M, shape.N);
+  // a policy that stores the result itself, or by rows, never uses the map, which still has to be
+  // a valid one
+  int rc = FRNNT_OK;
+  if (PairRowStore<Ext>::value)
+    mo = mah;
+  else if (Ext::kCustomStore)
+    rc = make_out_map(&mo, out, 1, 4, 4);
+  else
+    rc = make_out_map(&mo, out, shape.nz, shape.M, shape.N);
   if (rc != FRNNT_OK) return rc;
   auto kern = pair_umma_kernel<A_MN, B_MN, Ext>;
   FRNNT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemBytes));
@@ -490,7 +532,7 @@ int launch_pair_umma(const CUtensorMap &mah, const CUtensorMap &mal, const CUten
   rc = lin_grid((long long)shape.tiles_m * shape.tiles_n * shape.nz, &ctas);
   if (rc != FRNNT_OK) return rc;
   if (ctas == 0) return FRNNT_OK;
-  FRNNT_KERNEL(kern<<<ctas, kPairThreads, kPairSmemBytes, st>>>(mah, mal, mbh, mbl, mo, shape, ext));
+  FRNNT_KERNEL(kern<<<ctas, kPairThreads, kPairSmemBytes, st>>>(mah, mal, mbh, mbl, mo, out, shape, ext));
   FRNNT_CUDA(cudaGetLastError());
   return FRNNT_OK;
 }

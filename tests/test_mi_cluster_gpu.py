@@ -1,0 +1,67 @@
+"""The float lattice sweeps (csrc/mi_f32.cu) at the sizes where their split changes: one row per
+lane up to 32 lattice rows, two up to 64, a cluster of 2 .. 8 CTAs up to 512, row blocks
+beyond; chunks of 16 diagonals.  Tolerances are those of test_mi_gpu.py."""
+import random
+
+import pytest
+import torch
+
+from oracle import rnnt_oracle as orc
+from tests import workloads
+from tests.test_mi_gpu import assert_close
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(1, 1), (31, 16), (32, 17), (63, 15), (64, 97), (127, 130), (128, 144), (191, 200), (383, 40),
+         (511, 33), (512, 20), (1024, 50)]
+
+
+def run(px, py, bnd, w):
+    from fast_rnnt_b200 import mutual_information as mi
+    cb = None if bnd is None else bnd.cuda()
+    ans, _, lattice = mi.mi_forward(px.cuda(), py.cuda(), cb)
+    gx, gy = mi.mi_backward_from_lattice(px.cuda(), lattice, cb, w.cuda(), py.shape)
+    return ans.cpu(), gx.cpu(), gy.cpu()
+
+
+@pytest.mark.parametrize("modified", [False, True])
+@pytest.mark.parametrize("S,T", SIZES)
+def test_sweeps_at_the_edges_of_their_split(S, T, modified):
+    rng = random.Random(S)
+    torch.manual_seed(S + T)
+    B, T = 3, max(T, S) if modified else T
+    px = torch.rand(B, S, T + (0 if modified else 1)) * -4
+    py = torch.rand(B, S + 1, T) * -4
+    w = torch.linspace(0.5, 1.5, B)
+    for bnd in (None, workloads.random_mi_boundary(B, S, T, modified, rng)):
+        p, ans = orc.mi_forward_raw(px, py, bnd)
+        gx, gy = orc.mi_backward_raw(px, py, bnd, p, w)
+        got = run(px, py, bnd, w)
+        assert_close(got[0], ans, 1e-6, 1e-4, "ans")
+        # a chain of S + T cells of rounding up to 1e-4 each near a score of -2000
+        tol = 2e-5 if S + T < 700 else 1e-4
+        assert_close(got[1], gx, 0, tol, "px_grad")
+        assert_close(got[2], gy, 0, tol, "py_grad")
+
+
+@pytest.mark.parametrize("modified", [False, True])
+@pytest.mark.parametrize("S,T", [(20, 50), (40, 60), (100, 120)])
+def test_special_values_as_the_row_per_thread_sweeps(monkeypatch, S, T, modified):
+    torch.manual_seed(S)
+    lowest = torch.finfo(torch.float32).min
+    specials = [float("-inf"), float("inf"), float("nan"), lowest, -1e30, -1e6]
+    B = 2 * len(specials)
+    px = torch.rand(B, S, T + (0 if modified else 1)) * -4
+    py = torch.rand(B, S + 1, T) * -4
+    for i, v in enumerate(specials):
+        px[2 * i, S // 2, T // 3] = v
+        py[2 * i, S // 3, T // 2] = v
+        px[2 * i + 1, S // 2] = v      # every path meets it
+    w = torch.ones(B)
+    got = run(px, py, None, w)
+    monkeypatch.setenv("FRNNT_MI", "row_per_thread")
+    ref = run(px, py, None, w)
+    for a, b, what in zip(got, ref, ("ans", "px_grad", "py_grad")):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)), what
+        a, b = torch.nan_to_num(a, nan=0.0), torch.nan_to_num(b, nan=0.0)
+        assert_close(a, b, 2e-6, 2e-5, what)

@@ -1,0 +1,63 @@
+"""Simple lattices and their gradients on the tensor-core path for vocabularies that are no
+multiple of 4 and for tensors that are not 16-byte aligned, against the float64 path.
+
+The planes carry 22 bits of exp(x - max) in (0, 1], products accumulate in float32: 1e-5 on
+the lattices (scores up to 12: an ulp is 1e-6) and 2e-5 of the gradients' norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def lattices(lm, am, symbols, rnnt_type, scales, seed):
+    import fast_rnnt_b200 as fr
+    lm, am = lm.detach().requires_grad_(True), am.detach().requires_grad_(True)
+    px, py = fr.get_rnnt_logprobs_smoothed(lm, am, symbols, 0, lm_only_scale=scales[0],
+                                           am_only_scale=scales[1], rnnt_type=rnnt_type)
+    g = torch.Generator().manual_seed(seed)
+    gx = torch.rand(px.shape, generator=g).to(px)
+    gy = torch.rand(py.shape, generator=g).to(py)
+    gl, ga = torch.autograd.grad([px, py], [lm, am], [gx, gy])
+    return px.detach(), py.detach(), gl, ga
+
+
+@pytest.mark.parametrize("rnnt_type", ["regular", "modified", "constrained"])
+@pytest.mark.parametrize("C", [2, 3, 5, 50, 63, 65, 127, 129, 514, 4233])
+def test_odd_vocabulary_matches_float64(C, rnnt_type):
+    B, S, T = 2, 33, 131
+    torch.manual_seed(C)
+    lm, am = torch.randn(B, S + 1, C).cuda(), torch.randn(B, T, C).cuda()
+    symbols = torch.randint(1, C, (B, S)).cuda()
+    for scales in ((0.0, 0.0), (0.25, 0.1)):
+        got = lattices(lm, am, symbols, rnnt_type, scales, C)
+        ref = lattices(lm.double(), am.double(), symbols, rnnt_type, scales, C)
+        for a, b in zip(got[:2], ref[:2]):
+            fin = torch.isfinite(b)
+            assert torch.equal(torch.isfinite(a), fin)
+            assert float((a.double() - b)[fin].abs().max()) < 1e-5
+        for a, b in zip(got[2:], ref[2:]):
+            assert float((a.double() - b).norm()) < 2e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("C", [64, 65])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_unaligned_tensors(C, dtype):
+    B, S, T = 2, 9, 40
+    torch.manual_seed(C)
+    lm, am = torch.randn(B, S + 1, C).to(dtype).cuda(), torch.randn(B, T, C).to(dtype).cuda()
+    symbols = torch.randint(1, C, (B, S)).cuda()
+
+    def shifted(x):
+        flat = torch.empty(x.numel() + 1, dtype=x.dtype, device=x.device)
+        flat[1:] = x.reshape(-1)
+        return flat[1:].view(x.shape)
+
+    got = lattices(shifted(lm), shifted(am), symbols, "regular", (0.25, 0.0), C)
+    ref = lattices(lm.double(), am.double(), symbols, "regular", (0.25, 0.0), C)
+    for a, b in zip(got[:2], ref[:2]):
+        fin = torch.isfinite(b)
+        assert torch.equal(torch.isfinite(a), fin)
+        assert float((a.double() - b)[fin].abs().max()) < 1e-5
+    eps = 2e-5 if dtype == torch.float32 else float(torch.finfo(dtype).eps)
+    for a, b in zip(got[2:], ref[2:]):
+        assert float((a.double() - b).norm()) < eps * float(b.norm())
