@@ -5,6 +5,7 @@ is raised.  Tensors are passed as raw device pointers plus sizes; the current
 torch CUDA stream is passed to every call.
 """
 import ctypes
+import functools
 import os
 
 import torch
@@ -72,7 +73,38 @@ def ptr(t):
 
 
 def stream_ptr(device):
-    return _c_vp(torch.cuda.current_stream(device).cuda_stream)
+    """The current stream of the device, as the raw pointer torch keeps (no Stream object)."""
+    return _c_vp(torch._C._cuda_getCurrentRawStream(device.index))
+
+
+class _AlreadyCurrent:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_already_current = _AlreadyCurrent()
+
+
+def on_device(device):
+    """``torch.cuda.device(device)``, which costs several microseconds a use, only where the
+    device is not the current one already."""
+    if torch._C._cuda_getDevice() == device.index:
+        return _already_current
+    return torch.cuda.device(device)
+
+
+@functools.lru_cache(maxsize=1024)
+def _size_of(device: int, name: str, *args) -> int:
+    return int(getattr(lib(), name)(*args))
+
+
+def size_of(name: str, *args) -> int:
+    """Result of one of the pure size functions of the C ABI (buffer sizes from tensor sizes; some
+    depend on the current device's number of multiprocessors)."""
+    return _size_of(torch._C._cuda_getDevice(), name, *args)
 
 
 def check(rc: int, what: str):
@@ -82,5 +114,6 @@ def check(rc: int, what: str):
 
 
 def call(name: str, *args):
-    fn = getattr(lib(), name)
-    check(fn(*args), name)
+    rc = getattr(_lib or lib(), name)(*args)
+    if rc != 0:
+        check(rc, name)

@@ -19,7 +19,7 @@ def _matmul_tn(a, b, M, N, R, want_colsum=False):
     tiles as they pass through the product (the bias gradient of a linear layer)."""
     out = torch.empty(M, N, dtype=torch.float32, device=a.device)
     colsum = torch.empty(M, dtype=torch.float32, device=a.device) if want_colsum else None
-    nscratch = _lib.lib().frnnt_matmul_tn_scratch_floats(M, N, R)
+    nscratch = _lib.size_of("frnnt_matmul_tn_scratch_floats", M, N, R)
     scratch = torch.empty(max(nscratch, 1), dtype=torch.float32, device=a.device)
     _lib.call("frnnt_matmul_tn_colsum", _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(colsum),
               _lib.ptr(scratch), M, N, R, _lib.stream_ptr(a.device))
@@ -32,7 +32,7 @@ class _Linear3xTF32(torch.autograd.Function):
         N, K = weight.shape
         x2 = x.reshape(-1, K).contiguous()
         weight = weight.contiguous()
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x.device):
             out = _matmul_nt(x2, weight, None if bias is None else bias.contiguous(),
                              x2.shape[0], N, K)
         ctx.save_for_backward(x2, weight)
@@ -47,7 +47,7 @@ class _Linear3xTF32(torch.autograd.Function):
         M = x2.shape[0]
         g2 = g.reshape(M, N).contiguous()
         gx = gw = gb = None
-        with torch.cuda.device(g.device):
+        with _lib.on_device(g.device):
             if ctx.needs_input_grad[0]:
                 wt = weight.t().contiguous()                      # [K][N]
                 gx = _matmul_nt(g2, wt, None, M, K, N).reshape(ctx.x_shape)
@@ -83,7 +83,7 @@ class _PrunedJoiner(torch.autograd.Function):
         enc, dec, ranges, weight = (enc.contiguous(), dec.contiguous(), ranges.contiguous(),
                                     weight.contiguous())
         dev = enc.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             act = torch.empty(B, T, R, D, dtype=torch.float32, device=dev)
             _lib.call("frnnt_pruned_tanh", 0, _lib.ptr(enc), _lib.ptr(dec), _lib.ptr(ranges),
                       _lib.ptr(act), B, S1, T, R, D, _lib.stream_ptr(dev))
@@ -102,7 +102,7 @@ class _PrunedJoiner(torch.autograd.Function):
         dev = g.device
         g2 = g.reshape(M, N).contiguous()
         enc_grad = dec_grad = gw = gb = None
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
                 wt = weight.t().contiguous()
                 gz = _matmul_nt(g2, wt, None, M, D, N, tanh_out=act)   # d loss / d (enc + dec)
@@ -110,7 +110,7 @@ class _PrunedJoiner(torch.autograd.Function):
                 dec_grad = torch.empty(B, S1, D, dtype=torch.float32, device=dev)
                 if D % 4 == 0 and D <= 3200:
                     # both from one pass over gz
-                    nbytes = _lib.lib().frnnt_joiner_input_grads_scratch_bytes(B, T, D)
+                    nbytes = _lib.size_of("frnnt_joiner_input_grads_scratch_bytes", B, T, D)
                     scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
                     _lib.call("frnnt_joiner_input_grads", _lib.ptr(gz), _lib.ptr(ranges),
                               _lib.ptr(enc_grad), _lib.ptr(dec_grad), _lib.ptr(scratch), B, S1, T, R,

@@ -15,19 +15,34 @@ from . import _lib
 from ._lib import _c_int
 
 
-def _boundary_rows(boundary: Tensor):
-    """Host copy of the boundary rows, cached on the tensor so that the
-    validations along one loss call share a single device-to-host copy."""
+def _extremes(rows):
+    """What the range checks need of the boundary rows: (min s_begin, min s_end - s_begin,
+    max s_end, min t_begin, min t_end - t_begin, max t_end, min s_end, min t_end - s_end)."""
+    if not rows:
+        return (0, 0, 0, 0, 0, 0, 1, 0)
+    return (min(r[0] for r in rows), min(r[2] - r[0] for r in rows), max(r[2] for r in rows),
+            min(r[1] for r in rows), min(r[3] - r[1] for r in rows), max(r[3] for r in rows),
+            min(r[2] for r in rows), min(r[3] - r[2] for r in rows))
+
+
+def _host_copy(boundary: Tensor):
+    """(key, rows, extremes) of the boundary, kept on the tensor until it is modified, so that the
+    validations along one loss call share a single device-to-host copy and one pass over it."""
     key = (boundary.data_ptr(), boundary._version)
     cached = getattr(boundary, "_frnnt_rows", None)
     if cached is not None and cached[0] == key:
-        return cached[1]
+        return cached
     rows = boundary.tolist()
+    cached = (key, rows, _extremes(rows))
     try:
-        boundary._frnnt_rows = (key, rows)
+        boundary._frnnt_rows = cached
     except Exception:
         pass
-    return rows
+    return cached
+
+
+def _boundary_rows(boundary: Tensor):
+    return _host_copy(boundary)[1]
 
 
 def provide_boundary_rows(boundary: Tensor, rows) -> Tensor:
@@ -43,7 +58,7 @@ def provide_boundary_rows(boundary: Tensor, rows) -> Tensor:
     ``boundary``."""
     rows = rows.tolist() if isinstance(rows, Tensor) else [[int(v) for v in r] for r in rows]
     assert len(rows) == boundary.shape[0] and all(len(r) == 4 for r in rows)
-    boundary._frnnt_rows = ((boundary.data_ptr(), boundary._version), rows)
+    boundary._frnnt_rows = ((boundary.data_ptr(), boundary._version), rows, _extremes(rows))
     return boundary
 
 
@@ -55,14 +70,14 @@ def mi_forward(px: Tensor, py: Tensor, boundary: Optional[Tensor], want_p: bool 
     modified = int(T1 == T)
     dt = _lib.dtype_code(px.dtype)
     dev = px.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         ans = torch.empty(B, dtype=px.dtype, device=dev)
         p = torch.empty(B, S + 1, T + 1, dtype=px.dtype, device=dev) if want_p else None
         lattice = None
         # a lattice taller than one launch holds is swept in row blocks, which
         # hand the row above each block over through the scratch
-        if want_lattice or S + 1 > _lib.lib().frnnt_mi_rows_per_block(dt):
-            nbytes = _lib.lib().frnnt_mi_lattice_bytes(dt, B, S, T)
+        if want_lattice or S + 1 > _lib.size_of("frnnt_mi_rows_per_block", dt):
+            nbytes = _lib.size_of("frnnt_mi_lattice_bytes", dt, B, S, T)
             lattice = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
         _lib.call("frnnt_mi_forward", _c_int(dt), _lib.ptr(px), _lib.ptr(py), _lib.ptr(boundary),
                   _lib.ptr(p), _lib.ptr(ans), _lib.ptr(lattice), B, S, T, modified,
@@ -77,7 +92,7 @@ def mi_backward_from_lattice(px: Tensor, lattice: Tensor, boundary: Optional[Ten
     T = py_shape[2]
     modified = int(T1 == T)
     dev = px.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         px_grad = torch.empty_like(px)
         py_grad = torch.empty(py_shape, dtype=px.dtype, device=dev)
         _lib.call("frnnt_mi_backward_from_lattice", _c_int(_lib.dtype_code(px.dtype)),
@@ -96,8 +111,8 @@ def mi_backward_from_p(px: Tensor, py: Tensor, boundary: Optional[Tensor], p: Te
     modified = int(T1 == T)
     dt = _lib.dtype_code(px.dtype)
     dev = px.device
-    with torch.cuda.device(dev):
-        nbytes = _lib.lib().frnnt_mi_lattice_bytes(dt, B, S, T)
+    with _lib.on_device(dev):
+        nbytes = _lib.size_of("frnnt_mi_lattice_bytes", dt, B, S, T)
         lattice = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
         px_grad = torch.empty_like(px)
         py_grad = torch.empty_like(py)
@@ -167,9 +182,9 @@ def _validate(px: Tensor, py: Tensor, boundary: Optional[Tensor]):
     if boundary is not None:
         assert boundary.dtype == torch.int64
         assert boundary.shape == (B, 4)
-        for s_begin, t_begin, s_end, t_end in _boundary_rows(boundary):
-            assert 0 <= s_begin <= s_end <= S
-            assert 0 <= t_begin <= t_end <= T
+        s_begin, s_extent, s_end, t_begin, t_extent, t_end, _, _ = _host_copy(boundary)[2]
+        assert 0 <= s_begin and 0 <= s_extent and s_end <= S
+        assert 0 <= t_begin and 0 <= t_extent and t_end <= T
 
 
 def mutual_information_recursion(

@@ -21,7 +21,7 @@ from torch import Tensor
 
 from . import _lib
 from ._lib import _c_int, _c_f64
-from .mutual_information import _boundary_rows, mutual_information_recursion
+from .mutual_information import _boundary_rows, _host_copy, mutual_information_recursion
 
 _RNNT_TYPES = {"regular": 0, "modified": 1, "constrained": 2}
 
@@ -43,12 +43,10 @@ def validate_st_lengths(S: int, T: int, is_rnnt_type_regular: bool,
         assert (is_rnnt_type_regular or T >= S), \
             f"Modified transducer requires T >= S, but got T={T} and S={S}"
     else:
-        rows = _boundary_rows(boundary)
-        Ss = [r[2] for r in rows]
-        Ts = [r[3] for r in rows]
-        assert all(s >= 1 for s in Ss), Ss
-        assert (is_rnnt_type_regular or all(t >= s for s, t in zip(Ss, Ts))), \
-            f"Modified transducer requires T >= S, but got T={Ts} and S={Ss}"
+        _, rows, extremes = _host_copy(boundary)
+        assert extremes[6] >= 1, [r[2] for r in rows]
+        assert (is_rnnt_type_regular or extremes[7] >= 0), \
+            f"Modified transducer requires T >= S, but got T={[r[3] for r in rows]} and S={[r[2] for r in rows]}"
 
 
 def fix_for_boundary(px: Tensor, boundary: Optional[Tensor] = None) -> Tensor:
@@ -73,11 +71,11 @@ class _SimpleLogprobs(torch.autograd.Function):
         out_dtype = torch.float32 if _lib.is_16bit(lm) else lm.dtype
         T1 = T + 1 if rnnt_type == 0 else T
         lm, am, symbols, boundary = _contig(lm), _contig(am), _contig(symbols), _contig(boundary)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             px = torch.empty(B, S, T1, dtype=out_dtype, device=dev)
             py = torch.empty(B, S + 1, T, dtype=out_dtype, device=dev)
-            saved = _bytes(_lib.lib().frnnt_simple_saved_bytes(dt, B, S, T, C), dev)
-            scratch = _bytes(_lib.lib().frnnt_simple_scratch_bytes(dt, B, S, T, C), dev)
+            saved = _bytes(_lib.size_of("frnnt_simple_saved_bytes", dt, B, S, T, C), dev)
+            scratch = _bytes(_lib.size_of("frnnt_simple_scratch_bytes", dt, B, S, T, C), dev)
             _lib.call("frnnt_simple_logprobs_forward", _c_int(dt), _lib.ptr(lm), _lib.ptr(am),
                       _lib.ptr(symbols), _lib.ptr(boundary), blank, rnnt_type, int(smoothed),
                       _c_f64(ls), _c_f64(as_), _c_f64(delay_penalty), _lib.ptr(px), _lib.ptr(py),
@@ -95,14 +93,14 @@ class _SimpleLogprobs(torch.autograd.Function):
         dev, dt = lm.device, _lib.input_code(lm.dtype)
         out_dtype = torch.float32 if _lib.is_16bit(lm) else lm.dtype
         T1 = T + 1 if rnnt_type == 0 else T
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             g_px = (torch.zeros(B, S, T1, dtype=out_dtype, device=dev) if g_px is None
                     else g_px.contiguous())
             g_py = (torch.zeros(B, S + 1, T, dtype=out_dtype, device=dev) if g_py is None
                     else g_py.contiguous())
             lm_grad = torch.empty(lm.shape, dtype=out_dtype, device=dev)   # autograd casts it
             am_grad = torch.empty(am.shape, dtype=out_dtype, device=dev)
-            scratch = _bytes(_lib.lib().frnnt_simple_scratch_bytes(dt, B, S, T, C), dev)
+            scratch = _bytes(_lib.size_of("frnnt_simple_scratch_bytes", dt, B, S, T, C), dev)
             _lib.call("frnnt_simple_logprobs_backward", _c_int(dt), _lib.ptr(lm), _lib.ptr(am),
                       _lib.ptr(symbols), _lib.ptr(boundary), blank, rnnt_type, smoothed,
                       _c_f64(ls), _c_f64(as_), _lib.ptr(g_px), _lib.ptr(g_py), _lib.ptr(saved),
@@ -162,7 +160,7 @@ class _LsmGather(torch.autograd.Function):
         T1 = T + 1 if rnnt_type == 0 else T
         logits, symbols = _contig(logits), _contig(symbols)
         ranges, boundary = _contig(ranges), _contig(boundary)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             px = torch.empty(B, S, T1, dtype=logits.dtype, device=dev)
             py = torch.empty(B, S + 1, T, dtype=logits.dtype, device=dev)
             lse = torch.empty(3, B, T, R, dtype=logits.dtype, device=dev)
@@ -182,7 +180,7 @@ class _LsmGather(torch.autograd.Function):
         S = symbols.shape[1]
         dev, dt = logits.device, _lib.dtype_code(logits.dtype)
         T1 = T + 1 if rnnt_type == 0 else T
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             g_px = (torch.zeros(B, S, T1, dtype=logits.dtype, device=dev) if g_px is None
                     else g_px.contiguous())
             g_py = (torch.zeros(B, S + 1, T, dtype=logits.dtype, device=dev) if g_py is None
@@ -253,12 +251,11 @@ class _PrunedJoinerLogprobs(torch.autograd.Function):
         T1 = T + 1 if rnnt_type == 0 else T
         enc, dec, ranges, weight = _contig(enc), _contig(dec), _contig(ranges), _contig(weight)
         bias, symbols, boundary = _contig(bias), _contig(symbols), _contig(boundary)
-        lib = _lib.lib()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             px = torch.empty(B, S, T1, dtype=torch.float32, device=dev)
             py = torch.empty(B, S + 1, T, dtype=torch.float32, device=dev)
-            saved = _bytes(lib.frnnt_pruned_joiner_saved_bytes(B, T, R, S, C, D), dev)
-            scratch = _bytes(lib.frnnt_pruned_joiner_forward_scratch_bytes(B, T, R, S, C, D), dev)
+            saved = _bytes(_lib.size_of("frnnt_pruned_joiner_saved_bytes", B, T, R, S, C, D), dev)
+            scratch = _bytes(_lib.size_of("frnnt_pruned_joiner_forward_scratch_bytes", B, T, R, S, C, D), dev)
             _lib.call("frnnt_pruned_joiner_logprobs_forward", _c_int(_lib.input_code(enc.dtype)),
                       _lib.ptr(enc), _lib.ptr(dec),
                       _lib.ptr(ranges), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(symbols),
@@ -276,8 +273,7 @@ class _PrunedJoinerLogprobs(torch.autograd.Function):
         dev = saved.device
         T1 = T + 1 if rnnt_type == 0 else T
         need = ctx.needs_input_grad
-        lib = _lib.lib()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             g_px = (torch.zeros(B, S, T1, dtype=torch.float32, device=dev) if g_px is None
                     else g_px.contiguous())
             g_py = (torch.zeros(B, S + 1, T, dtype=torch.float32, device=dev) if g_py is None
@@ -288,7 +284,7 @@ class _PrunedJoinerLogprobs(torch.autograd.Function):
             w_grad = torch.empty(C, D, dtype=torch.float32, device=dev) if need[3] else None
             b_grad = (torch.empty(C, dtype=torch.float32, device=dev)
                       if has_bias and need[4] else None)
-            scratch = _bytes(lib.frnnt_pruned_joiner_backward_scratch_bytes(B, T, R, S, C, D), dev)
+            scratch = _bytes(_lib.size_of("frnnt_pruned_joiner_backward_scratch_bytes", B, T, R, S, C, D), dev)
             _lib.call("frnnt_pruned_joiner_logprobs_backward", _lib.ptr(g_px), _lib.ptr(g_py),
                       _lib.ptr(ranges), _lib.ptr(symbols), _lib.ptr(boundary), _lib.ptr(saved),
                       _lib.ptr(scratch), _lib.ptr(enc_grad), _lib.ptr(dec_grad), _lib.ptr(w_grad),
@@ -378,7 +374,7 @@ def get_rnnt_prune_ranges(px_grad: Tensor, py_grad: Tensor, boundary: Tensor,
 
     dev = px_grad.device
     px_grad, py_grad, boundary = px_grad.contiguous(), py_grad.contiguous(), boundary.contiguous()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         ranges = torch.empty(B, T, s_range, dtype=torch.int64, device=dev)
         _lib.call("frnnt_prune_ranges", _c_int(_lib.dtype_code(px_grad.dtype)),
                   _lib.ptr(px_grad.detach()), _lib.ptr(py_grad.detach()), _lib.ptr(boundary),
@@ -393,7 +389,7 @@ class _PruneGather(torch.autograd.Function):
         _, T, R = ranges.shape
         dev = lm.device
         lm, ranges = lm.contiguous(), ranges.contiguous()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             out = torch.empty(B, T, R, D, dtype=lm.dtype, device=dev)
             _lib.call("frnnt_prune_gather", _c_int(_lib.dtype_code(lm.dtype)), _lib.ptr(lm),
                       _lib.ptr(ranges), _lib.ptr(out), B, S1, T, R, D, _lib.stream_ptr(dev))
@@ -408,11 +404,11 @@ class _PruneGather(torch.autograd.Function):
         _, T, R = ranges.shape
         dev = g.device
         g = g.contiguous()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             lm_grad = torch.empty(B, S1, D, dtype=g.dtype, device=dev)
             if g.dtype == torch.float32 and D % 4 == 0 and D <= 3200:
                 # windowed partial sums per chunk of frames (one streaming pass)
-                nbytes = _lib.lib().frnnt_joiner_input_grads_scratch_bytes(B, T, D)
+                nbytes = _lib.size_of("frnnt_joiner_input_grads_scratch_bytes", B, T, D)
                 scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
                 _lib.call("frnnt_joiner_input_grads", _lib.ptr(g), _lib.ptr(ranges), None,
                           _lib.ptr(lm_grad), _lib.ptr(scratch), B, S1, T, R, D,
