@@ -24,9 +24,9 @@
 //     reads are contiguous row segments, ring reads by the diagonal are
 //     bank-conflict free (pitch 33);
 //   * the forward sweep stores, by anti-diagonal in a scratch ("lattice", fully
-//     coalesced), the exponent of the backward weight of every cell,
+//     coalesced; float: through exp already), the exponent of every cell's backward weight,
 //     p[s-1][t+o] + px[s-1][t+o] - p[s][t], which it has in registers anyway.  In
-//     the backward sweep the helper warps turn it into the weights d1 (the only
+//     the backward sweep the helper warps turn it into the weights d1 (double: the only
 //     exp() of the backward) one chunk ahead of the compute warps, whose
 //     dependent chain per step is shuffle + add + multiply;
 //   * gradients leave through the same kind of skewed ring, written back as
@@ -281,7 +281,7 @@ mi_forward_kernel(const real *__restrict__ px, const real *__restrict__ py,
         if (L != nullptr) {
 #pragma unroll
           for (int u = 0; u < 8; ++u)
-            if (act_mask >> u & 1u) L[(size_t)u * lpitch] = dlv[u];
+            if (act_mask >> u & 1u) L[(size_t)u * lpitch] = lattice_value(dlv[u]);
           L += (size_t)8 * lpitch;
         }
         if (BLOCKED && i == ROWS - 1) {
@@ -410,8 +410,8 @@ mi_backward_kernel(const real *__restrict__ px, real *__restrict__ lattice,
             d1 = MODIFIED ? 0 : 1;
           } else {
             // an unreachable cell has a non-finite exponent; it gets no gradient
-            const real w = exp_r(dl[jj][m]);
-            if (w - w == 0) {
+            const real w = weight_of(dl[jj][m]);
+            if (w - w == 0 && w >= 0) {
               d1 = w;
               d2 = (real)1 - w;
             }
@@ -543,14 +543,12 @@ mi_backward_kernel(const real *__restrict__ px, real *__restrict__ lattice,
   }
 }
 
-// p in the reference's [B][S+1][T+1] layout -> the weight exponents
-// p[s-1][t+o] + px[s-1][t+o] - p[s][t] in the diagonal-major scratch, or (as_weights) the weights
-// themselves as the sweeps of mi_f32.cu keep them
+// p in the reference's [B][S+1][T+1] layout -> what the forward sweep leaves in the diagonal-major
+// scratch
 template <typename real>
 __global__ void mi_lattice_from_p_kernel(const real *__restrict__ p, const real *__restrict__ px,
                                          const int64_t *__restrict__ boundary,
-                                         real *__restrict__ lattice, int S, int T, int modified,
-                                         int as_weights) {
+                                         real *__restrict__ lattice, int S, int T, int modified) {
   const int b = blockIdx.y;
   const MiBox box = load_box(boundary, b, S, T);
   const int T1 = modified ? T : T + 1, off = modified ? -1 : 0;
@@ -563,15 +561,11 @@ __global__ void mi_lattice_from_p_kernel(const real *__restrict__ p, const real 
        idx += gridDim.x * blockDim.x) {
     const int i = idx / (box.tb + 1), tp = idx % (box.tb + 1);
     real d = 0;  // first row / first column: the weights are fixed by position
-    if (as_weights && i >= 1 && tp == 0) d = modified ? kMiDead : 1;
     if (i >= 1 && tp >= 1) {
       const size_t up = (size_t)(box.s0 + i - 1);
       d = P[up * (T + 1) + box.t0 + tp + off] + X[up * T1 + box.t0 + tp + off] -
           P[(size_t)(box.s0 + i) * (T + 1) + box.t0 + tp];
-      if (as_weights) {
-        d = exp_r(d);
-        if (!(d - d == 0)) d = kMiDead;
-      }
+      d = lattice_value(d);
     }
     LT[(size_t)(i + tp) * lpitch + i] = d;
   }
@@ -821,11 +815,10 @@ extern "C" int frnnt_mi_backward(int dtype, const void *px, const void *py,
   dim3 grid((unsigned)min(64, ((S + 1) * (T + 1) + 255) / 256), (unsigned)B);
   if (dtype == FRNNT_F32)
     FRNNT_KERNEL(mi_lattice_from_p_kernel<float><<<grid, 256, 0, st>>>(
-        (const float *)p, (const float *)px, boundary, (float *)lattice, S, T, modified,
-        mi_use_f32(dtype, lattice)));
+        (const float *)p, (const float *)px, boundary, (float *)lattice, S, T, modified));
   else
     FRNNT_KERNEL(mi_lattice_from_p_kernel<double><<<grid, 256, 0, st>>>(
-        (const double *)p, (const double *)px, boundary, (double *)lattice, S, T, modified, 0));
+        (const double *)p, (const double *)px, boundary, (double *)lattice, S, T, modified));
   FRNNT_CUDA(cudaGetLastError());
   return frnnt_mi_backward_from_lattice(dtype, px, lattice, boundary, ans_grad, px_grad, py_grad,
                                         origin_grad, B, S, T, modified, stream);

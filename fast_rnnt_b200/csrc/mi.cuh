@@ -50,10 +50,23 @@ __device__ __forceinline__ void bar_sync_named(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// What the lattice scratch holds of a cell: double the exponent of its backward weight (share of
+// the x-predecessor), p[s-1][t+o] + px[s-1][t+o] - p[s][t]; float the weight itself, or kMiDead
+// where the exponent is not finite (no path reaches the cell; it passes no gradient on).
+constexpr float kMiDead = -1.f;
+__device__ __forceinline__ float mi_weight(float exponent) {
+  const float w = expf(exponent);
+  return w - w == 0.f ? w : kMiDead;
+}
+__device__ __forceinline__ float lattice_value(float exponent) { return mi_weight(exponent); }
+__device__ __forceinline__ double lattice_value(double exponent) { return exponent; }
+// weight from what the lattice holds; not finite or negative: no gradient
+__device__ __forceinline__ float weight_of(float value) { return value; }
+__device__ __forceinline__ double weight_of(double value) { return exp(value); }
+
 // float sweeps (mi_f32.cu).  `lattice` must be 16-byte aligned; the forward takes NULL when
 // the whole lattice fits one launch (S + 1 <= kMiF32Rows) and no backward sweep follows.
 constexpr int kMiF32Rows = 512;
-constexpr float kMiDead = -1.f;  // their weight of a cell outside the box, or that no path reaches
 int launch_mi_forward_f32(const float *px, const float *py, const int64_t *boundary, float *p, float *ans,
                           float *lattice, int B, int S, int T, int modified, cudaStream_t st);
 int launch_mi_backward_f32(float *lattice, const int64_t *boundary, const float *ans_grad, float *px_grad,

@@ -116,7 +116,7 @@ __device__ __forceinline__ void peer_send(unsigned address, float v, unsigned ba
 }
 
 // Hand-over of the edge row between neighbouring CTAs, chunks numbered in the order of the sweep.
-// Each side has one mbarrier per slot of the edge ring (chunk mod 4): `full` in the consumer's
+// Each side has one mbarrier per slot of the edge ring (chunk mod 8): `full` in the consumer's
 // shared memory, `taken` in the producer's.  Every wait is bounded; one that runs out makes
 // all later ones give up at once (and the caller's results NaN).
 constexpr int kSlots = kEdgeRing / kStep;
@@ -278,12 +278,7 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
       float w[4];
       load_rows<4>(w, ringw + ((c & 1) * kStep + j) * PITCH + l0);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        w[r] = expf(w[r]);
-        if (!(w[r] - w[r] == 0.f)) w[r] = kMiDead;                // nothing reaches this cell
-        if (k - q0 - r == 0) w[r] = MODIFIED ? kMiDead : 1.f;     // first column: only an x-predecessor
-        if (r == 0 && row0 + q0 == 0) w[r] = 0.f;                 // first row: only a y-predecessor
-      }
+      for (int r = 0; r < 4; ++r) w[r] = mi_weight(w[r]);
       store_rows<4>(L + (size_t)k * lpitch + q0, w);
     }
   };
@@ -487,10 +482,14 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
       const int q = (n * kHelpers + hw) * 32 + lane;
       const int l0 = 4 * (q % (ROWS / 4)), j = q / (ROWS / 4);
       const int tp0 = chunk_of(it) * kStep + j - first - l0;
-      // what the lattice holds outside the box is not defined
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < 4; ++r) {
+        // first column: only an x-predecessor (regular) or none; first row: only a y-predecessor;
+        // what the lattice holds outside the box is not defined
+        if (tp0 - r == 0) wv[n][r] = MODIFIED ? kMiDead : 1.f;
+        if (r == 0 && row0 + first + l0 == 0) wv[n][r] = 0.f;
         if (first + l0 + r > ib || (unsigned)(tp0 - r) > (unsigned)box.tb) wv[n][r] = kMiDead;
+      }
       if (q < M::kQuads) store_rows<4>(ringw + ((it & 1) * kStep + j) * PITCH + l0, wv[n]);
     }
     if (BLOCKED && rank == ranks - 1 && hw == 0 && lane < kStep)

@@ -65,3 +65,18 @@ def test_special_values_as_the_row_per_thread_sweeps(monkeypatch, S, T, modified
         assert torch.equal(torch.isnan(a), torch.isnan(b)), what
         a, b = torch.nan_to_num(a, nan=0.0), torch.nan_to_num(b, nan=0.0)
         assert_close(a, b, 2e-6, 2e-5, what)
+
+
+@pytest.mark.parametrize("S,T", [(20, 40), (100, 70)])
+def test_scratch_off_a_16_byte_boundary(S, T):
+    """Both families of float sweeps keep the same scratch: an unaligned copy takes the other one."""
+    from fast_rnnt_b200 import mutual_information as mi
+    torch.manual_seed(S)
+    px, py = (torch.rand(2, S, T + 1) * -4).cuda(), (torch.rand(2, S + 1, T) * -4).cuda()
+    w = torch.ones(2).cuda()
+    _, _, lattice = mi.mi_forward(px, py, None)
+    moved = torch.empty(lattice.numel() + 4, dtype=torch.uint8, device="cuda")[4:]
+    moved.copy_(lattice)
+    for a, b in zip(mi.mi_backward_from_lattice(px, lattice, None, w, py.shape),
+                    mi.mi_backward_from_lattice(px, moved, None, w, py.shape)):
+        assert torch.equal(a, b)
