@@ -141,6 +141,7 @@ __global__ void column_partial_kernel(const real *__restrict__ x, const real *__
   const long long r0 = (long long)blockIdx.y * kColChunkRows;
   const long long r1 = min(rows, r0 + kColChunkRows);
   real acc = 0;
+#pragma unroll 8
   for (long long r = r0; r < r1; ++r) {
     const real e = exp_r(x[r * C + c] - rmax[r]);
     if (MODE == 0) {
@@ -159,6 +160,7 @@ __global__ void unigram_final_kernel(const real *__restrict__ partial, int nchun
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   real acc = 0;
+#pragma unroll 8
   for (int j = 0; j < nchunk; ++j) acc += partial[(size_t)j * C + c];
   const real u = acc / (real)rows + tiny_v<real>();
   uni[c] = u;
@@ -177,6 +179,7 @@ __global__ void am_only_norm_kernel(const real *__restrict__ am, const real *__r
     const real *src = am + row * (long long)C;
     const real m = ammax[row];
     real z = 0;
+#pragma unroll 8
     for (int c = lane; c < C; c += 32) z += exp_r(src[c] - m) * uni[c];
     z = warp_sum(z);
     if (lane == 0) amonly[row] = log_r(z) + m;
@@ -677,6 +680,7 @@ __global__ void row_dot_kernel(const real *__restrict__ lm, const real *__restri
   const real *src = lm + row * (long long)C;
   const real m = lmmax[row];
   real acc = 0;
+#pragma unroll 8
   for (int c = lane; c < C; c += 32) acc += exp_r(src[c] - m) * dp[c];
   acc = warp_sum(acc);
   if (lane == 0) rowdot[row] = acc / lmsum[row];

@@ -73,7 +73,7 @@ bool simple_pairs_supported(const void *lm, const void *am, int S1, int T, int C
 // Four entries of a row at a time as one 16-byte (8-byte) load, TMA stores of the gradients: for
 // vocabularies that are a multiple of 4 and 16-byte aligned tensors.  Everything else reads
 // single entries and stores gradient boxes row by row.  16 x (59, 293) x 4233, forward and
-// backward: normalizer 76, lm / am gradient 52 / 90, planes 74 us, against 1503, 294 / 248 and
+// backward: normalizer 76, lm / am gradient 52 / 90, planes 40 us, against 1503, 294 / 248 and
 // 48 us on the FMA pipe.
 static bool rows_by_four(const void *a, const void *b, int C) {
   return C % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)b % 16 == 0;
@@ -89,8 +89,12 @@ __device__ __forceinline__ float4 row_load4(const TIn *row, int v, int C) {
                      c + 2 < C ? in_f32(row[c + 2]) : -INFINITY, c + 3 < C ? in_f32(row[c + 3]) : -INFINITY);
 }
 
-// one warp per row of lm (rows 0 .. B*S1-1) or am (the rest)
-template <typename TIn, bool VEC>
+// G warps per row of lm (rows 0 .. B*S1-1) or am (the rest), each lane keeping K vectors of four
+// entries: a row of up to 128 G K entries is read once.  What bounds the kernel is HBM (read
+// 4 C, write 4 C bytes a row); re-reading what one warp cannot keep made rows of 5000 entries
+// take 1.5 times as long (64 x (60, 400) x 5000: 312 -> 208 us, 157 at the copy rate;
+// 16 x (59, 293) x 4233, single entries: 74 -> 40 us).
+template <typename TIn, bool VEC, int G, int K>
 __global__ void __launch_bounds__(256)
 exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
                   const int64_t *__restrict__ symbols, __half *__restrict__ lp_hi,
@@ -99,33 +103,48 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
                   float *__restrict__ lm_blk, float *__restrict__ lm_sym, float *__restrict__ lnorm,
                   float *__restrict__ am_blk, float *__restrict__ am_sym, float *__restrict__ px, int B,
                   int S, int T, int C, int Cp, int Sp, int blank, int regular) {
-  const int lane = threadIdx.x & 31;
-  const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  constexpr int LANES = 32 * G, RPB = 8 / G;  // threads of a row, rows of a CTA
+  __shared__ float part[8];
+  const int lane = threadIdx.x % LANES, slot = threadIdx.x / LANES;
   const int S1 = S + 1, nvec = (C + 3) / 4;
   const long long rows_lm = (long long)B * S1, rows = rows_lm + (long long)B * T;
-  for (long long row = warp0; row < rows; row += nwarps) {
+  auto over_group = [&](float v, bool is_max) {
+    v = is_max ? warp_max(v) : warp_sum(v);
+    if (G > 1) {
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+      __syncthreads();
+      v = part[slot * G];
+#pragma unroll
+      for (int w = 1; w < G; ++w) v = is_max ? fmaxf(v, part[slot * G + w]) : v + part[slot * G + w];
+    }
+    return v;
+  };
+  for (long long row0 = (long long)blockIdx.x * RPB; row0 < rows; row0 += (long long)gridDim.x * RPB) {
+    // a CTA's last rows may not exist; they take part in the barriers of the others
+    const bool valid = row0 + slot < rows;
+    if (G == 1 && !valid) break;
+    const long long row = valid ? row0 + slot : rows - 1;
     const bool is_lm = row < rows_lm;
     const long long r = is_lm ? row : row - rows_lm;
     const TIn *src = (is_lm ? lm : am) + r * C;
     uint2 *dh = reinterpret_cast<uint2 *>((is_lm ? lp_hi : ap_hi) + r * Cp);
     uint2 *dl = reinterpret_cast<uint2 *>((is_lm ? lp_lo : ap_lo) + r * Cp);
-    // the first four vectors of a lane stay in registers (rows up to 512 entries are read once)
-    float4 keep[4];
+    float4 keep[K];
     float m = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int v = lane + 32 * j;
-      if (v < nvec) {
-        keep[j] = row_load4<VEC>(src, v, C);
-        m = fmaxf(fmaxf(m, fmaxf(keep[j].x, keep[j].y)), fmaxf(keep[j].z, keep[j].w));
-      }
+    for (int j = 0; j < K; ++j) {
+      const int v = lane + LANES * j;
+      if (v < nvec) keep[j] = row_load4<VEC>(src, v, C);
     }
-    for (int v = lane + 128; v < nvec; v += 32) {
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      if (lane + LANES * j < nvec) m = fmaxf(fmaxf(m, fmaxf(keep[j].x, keep[j].y)), fmaxf(keep[j].z, keep[j].w));
+    for (int v = lane + LANES * K; v < nvec; v += LANES) {
       const float4 q = row_load4<VEC>(src, v, C);
       m = fmaxf(fmaxf(m, fmaxf(q.x, q.y)), fmaxf(q.z, q.w));
     }
-    m = warp_max(m);
+    m = over_group(m, true);
     float sum = 0.f;
     auto one = [&](int v, const float4 &q) {
       const float e[4] = {expf(q.x - m), expf(q.y - m), expf(q.z - m), expf(q.w - m)};
@@ -133,23 +152,23 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
       for (int i = 0; i < 4; ++i) sum += e[i];
       uint2 hi, lo;
       fp16_pair4(e, kExpScale, hi, lo);
-      dh[v] = hi;
-      dl[v] = lo;
+      if (valid) dh[v] = hi, dl[v] = lo;
     };
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int v = lane + 32 * j;
+    for (int j = 0; j < K; ++j) {
+      const int v = lane + LANES * j;
       if (v < nvec) one(v, keep[j]);
     }
-    for (int v = lane + 128; v < nvec; v += 32) one(v, row_load4<VEC>(src, v, C));
-    sum = warp_sum(sum);
+    for (int v = lane + LANES * K; v < nvec; v += LANES) one(v, row_load4<VEC>(src, v, C));
+    sum = over_group(sum, false);
+    if (!valid) continue;
     if (!is_lm) {
       // am[t][symbol of every lattice row]: gathered here, where the row has just been read
       // (L1 hits), so that the product's epilogue reads them as whole 128-byte lines
       const TIn *x = am + r * C;
       const int64_t *sy = symbols + (size_t)div_rows(r, T) * S;
       float *dst = am_sym + (size_t)r * Sp;
-      for (int s = lane; s < Sp; s += 32) {
+      for (int s = lane; s < Sp; s += LANES) {
         float v = 0.f;
         if (s < S) {
           long long y = sy[s];
@@ -446,20 +465,33 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
   const int S1 = S + 1;
   if (stage == 0) {
     const long long rows = (long long)B * (S1 + T);
-    long long want = (rows + 7) / 8;
-    const int grid = (int)(want < (long long)sm_count() * 32 ? want : (long long)sm_count() * 32);
     const bool vec = rows_by_four(lm, am, C);
-#define FRNNT_EXP_PLANES_AS(TIn, VEC)                                                                                   \
-  FRNNT_KERNEL(exp_planes_kernel<TIn, VEC><<<grid, 256, 0, st>>>((const TIn *)lm, (const TIn *)am, symbols, lp_hi, lp_lo,  \
-                                                           ap_hi, ap_lo, lmmax, lmsum, ammax, lm_blk, lm_sym, lnorm, \
-                                                           am_blk, am_sym, px, B, S, T, C, L.Cp, L.Sp, blank,        \
-                                                           rnnt_type == FRNNT_REGULAR))
-#define FRNNT_EXP_PLANES(TIn)          \
-  do {                                 \
-    if (vec)                           \
-      FRNNT_EXP_PLANES_AS(TIn, true);  \
-    else                               \
-      FRNNT_EXP_PLANES_AS(TIn, false); \
+    // lanes keep 16 entries in rows up to 512, else 32, with as many warps as that takes
+#define FRNNT_EXP_PLANES_AS(TIn, VEC, G, K)                                                                         \
+  FRNNT_KERNEL(exp_planes_kernel<TIn, VEC, G, K>                                                                    \
+               <<<(int)std::min<long long>((rows * G + 7) / 8, (long long)sm_count() * 32), 256, 0, st>>>(          \
+                   (const TIn *)lm, (const TIn *)am, symbols, lp_hi, lp_lo, ap_hi, ap_lo, lmmax, lmsum, ammax,      \
+                   lm_blk, lm_sym, lnorm, am_blk, am_sym, px, B, S, T, C, L.Cp, L.Sp, blank,                        \
+                   rnnt_type == FRNNT_REGULAR))
+#define FRNNT_EXP_PLANES_BY(TIn, VEC)       \
+  do {                                      \
+    if (C <= 512)                           \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 4);  \
+    else if (C <= 1024)                     \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 8);  \
+    else if (C <= 2048)                     \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 2, 8);  \
+    else if (C <= 4096)                     \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 4, 8);  \
+    else                                    \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 8, 8);  \
+  } while (0)
+#define FRNNT_EXP_PLANES(TIn)            \
+  do {                                   \
+    if (vec)                             \
+      FRNNT_EXP_PLANES_BY(TIn, true);    \
+    else                                 \
+      FRNNT_EXP_PLANES_BY(TIn, false);   \
   } while (0)
     if (input_dtype == FRNNT_F16) {
       FRNNT_EXP_PLANES(__half);
@@ -469,6 +501,7 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
       FRNNT_EXP_PLANES(float);
     }
 #undef FRNNT_EXP_PLANES
+#undef FRNNT_EXP_PLANES_BY
 #undef FRNNT_EXP_PLANES_AS
     FRNNT_CUDA(cudaGetLastError());
     return FRNNT_OK;

@@ -22,7 +22,7 @@ def lattices(lm, am, symbols, rnnt_type, scales, seed):
 
 
 @pytest.mark.parametrize("rnnt_type", ["regular", "modified", "constrained"])
-@pytest.mark.parametrize("C", [2, 3, 5, 50, 63, 65, 127, 129, 514, 4233])
+@pytest.mark.parametrize("C", [2, 3, 5, 50, 63, 65, 127, 129, 514, 1024, 1025, 2049, 4096, 4233, 8193])
 def test_odd_vocabulary_matches_float64(C, rnnt_type):
     B, S, T = 2, 33, 131
     torch.manual_seed(C)
