@@ -83,14 +83,16 @@ int frnnt_with_cuda(void);
  * ------------------------------------------------------------------------- */
 
 /* Bytes of the `lattice` scratch of the functions below: the forward sweep
- * stores there, by anti-diagonal ([B][S+T+1][round_up(S+1,32)]), the exponent of
- * every cell's backward weight, p[s-1][t+o] + px[s-1][t+o] - p[s][t], so that it
- * writes it and the backward sweep reads it fully coalesced; two vectors of
- * S+T+65 values per utterance follow (see frnnt_mi_rows_per_block). */
+ * stores there, by anti-diagonal ([B][S+T+1][round_up(S+1,32)]), every cell's
+ * backward weight (FRNNT_F32) or its exponent (FRNNT_F64),
+ * p[s-1][t+o] + px[s-1][t+o] - p[s][t], so that it writes it and the backward sweep
+ * reads it fully coalesced; two vectors of S+T+65 values per utterance follow
+ * (see frnnt_mi_rows_per_block). */
 size_t frnnt_mi_lattice_bytes(int dtype, int B, int S, int T);
 
-/* Lattice rows (S+1) that one launch sweeps: 256 for FRNNT_F32, 128 for
- * FRNNT_F64.  A taller lattice is swept in blocks of that many rows, one launch
+/* Lattice rows (S+1) up to which a forward sweep alone needs no scratch: 256 for
+ * FRNNT_F32, 128 for FRNNT_F64.  A taller lattice (FRNNT_F32: taller than the
+ * 512 rows of a cluster) is swept in blocks of rows, one launch
  * per block and direction (the reference tiles in 32x32 blocks and launches once
  * per anti-diagonal of tiles, mutual_information_cuda.cu:680-731).  The row above
  * a block and the gradients that cross a block edge travel from launch to launch
