@@ -25,10 +25,6 @@
 //     sends the edge row;
 //   * cells outside the box need no test in the forward chain: they are fed x = -inf, y = 0,
 //     which keeps rows that have not begun at -inf and the origin at 0;
-//   * LogAdd is hi + log1p(e), e = exp(-|a - b|), both written out for the range that occurs
-//     (one ex2.approx and a polynomial; no branch).  Operands whose difference is not finite,
-//     or too large for e to count, give hi itself, the guard of the reference's LogAdd
-//     (fast_rnnt/csrc/mutual_information.h:36-65);
 //   * the forward's helpers turn the exponents a - p[s][t] that its compute warp leaves in
 //     shared memory into the backward weights (kMiDead: a cell that passes no gradient on), so
 //     that the helpers of the backward only copy them in and the gradients out.
@@ -44,17 +40,6 @@ constexpr int kThreads = 256;
 constexpr int kEdgeRing = 128;  // edge-row values kept (eight chunks)
 constexpr int kMaxCluster = 8;
 
-// (log1p(e) - e) / e^2 on [0, 1] as a polynomial in e - 1/2 (minimax fit by Lawson iteration,
-// rounded to float32).  log1p(e) = e + e^2 r(e) then has an absolute error of at most 7.0e-8,
-// 9.6e-9 on average over [0, 1] (a correctly rounded result: 3.0e-8 at most).
-__device__ __forceinline__ float log1p_unit(float e) {
-  const float z = e - 0.5f, z2 = z * z, z4 = z2 * z2;
-  const float q01 = fmaf(0.179224819f, z, -0.378139555f), q23 = fmaf(0.0510927849f, z, -0.0932318643f);
-  const float q45 = fmaf(0.0166102126f, z, -0.0289093703f), q67 = fmaf(0.00708867516f, z, -0.0101047074f);
-  const float q03 = fmaf(q23, z2, q01), q48 = fmaf(-0.00359314145f, z4, fmaf(q67, z2, q45));
-  return fmaf(e * e, fmaf(q48, z4, q03), e);
-}
-
 // if (cond) acc = x + y, as one predicated instruction (a select would lengthen the chain)
 __device__ __forceinline__ void add_if(float &acc, bool cond, float x, float y) {
   asm("{\n.reg .pred q;\nsetp.ne.s32 q, %3, 0;\n@q add.f32 %0, %1, %2;\n}"
@@ -62,16 +47,15 @@ __device__ __forceinline__ void add_if(float &acc, bool cond, float x, float y) 
       : "f"(x), "f"(y), "r"((int)cond));
 }
 
+// LogAdd with the values of log_add(): a difference that is not finite, or too large for exp()
+// to count, leaves the larger operand.  expf and log1pf are the library's on purpose: a faster
+// pair (one ex2 and a polynomial of the same error, 0.7 of this kernel's time) rounds a few
+// cells in a thousand to a neighbouring float32, and prune ranges are an argmax that such
+// neighbours can move.
 __device__ __forceinline__ float log_add_f32(float a, float b) {
-  constexpr float kLog2e = 1.44269504f, kLn2 = 0.693147181f;
-  const bool less = a < b;
-  const float d = a - b, t = d * kLog2e;
-  // what the rounding of the product left out of the exponent -|t|
-  const float rest = fmaf(d, kLog2e, -t) * (less ? kLn2 : -kLn2);
-  float e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-fabsf(t)));
-  float r = less ? b : a;
-  add_if(r, fabsf(d) < 150.f, r, log1p_unit(fmaf(e, rest, e)));
+  const float d = a - b;
+  float r = a < b ? b : a;
+  add_if(r, fabsf(d) < 150.f, r, log1pf(expf(-fabsf(d))));
   return r;
 }
 

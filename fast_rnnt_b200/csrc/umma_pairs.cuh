@@ -42,7 +42,8 @@
 //                                                  staging and the TMA store, for the 32-column
 //                                                  boxes of a tile from the last to the first
 //   static constexpr int kGroup;                   (optional, default kPairGroup) K slices per
-//                                                  accumulator group
+//                                                  accumulator group; below the default the small
+//                                                  products of a slice come first, too (accuracy)
 //   static constexpr bool kRowStore;               (optional, default false) boxes leave by coalesced
 //                                                  stores, a row segment each, instead of TMA: outputs
 //                                                  whose rows are not a multiple of 16 bytes
@@ -306,15 +307,28 @@ pair_umma_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
           tc_fence_after_sync();
           const uint32_t acc = tmem_d + ((gg & 1) ? kPairAcc1 : 0u);
           const uint32_t st = tiles + (uint32_t)s * kPairStageBytes;
-          // the small products first: what the accumulator cuts off when it adds scales with what
-          // it holds by then
+          if (GROUP < kPairGroup) {
+            // the small products first: what the accumulator cuts off when it adds scales with
+            // what it holds by then
 #pragma unroll
-          for (int q = 0; q < 3; ++q) {
+            for (int q = 0; q < 3; ++q) {
+#pragma unroll
+              for (int ks = 0; ks < kPairBK / 16; ++ks) {
+                const uint64_t da = smem_desc_sw128(st + (q == 0 ? kPairOpBytes : 0) + ks * a_step, a_lbo, 1024u);
+                const uint64_t db = smem_desc_sw128(st + (q == 1 ? 3 : 2) * kPairOpBytes + ks * b_step, b_lbo, 1024u);
+                mma_f16_ss(acc, da, db, idesc, (!group_start || q > 0 || ks > 0) ? 1u : 0u);
+              }
+            }
+          } else {
 #pragma unroll
             for (int ks = 0; ks < kPairBK / 16; ++ks) {
-              const uint64_t da = smem_desc_sw128(st + (q == 0 ? kPairOpBytes : 0) + ks * a_step, a_lbo, 1024u);
-              const uint64_t db = smem_desc_sw128(st + (q == 1 ? 3 : 2) * kPairOpBytes + ks * b_step, b_lbo, 1024u);
-              mma_f16_ss(acc, da, db, idesc, (!group_start || q > 0 || ks > 0) ? 1u : 0u);
+              const uint64_t dah = smem_desc_sw128(st + ks * a_step, a_lbo, 1024u);
+              const uint64_t dal = smem_desc_sw128(st + kPairOpBytes + ks * a_step, a_lbo, 1024u);
+              const uint64_t dbh = smem_desc_sw128(st + 2 * kPairOpBytes + ks * b_step, b_lbo, 1024u);
+              const uint64_t dbl = smem_desc_sw128(st + 3 * kPairOpBytes + ks * b_step, b_lbo, 1024u);
+              mma_f16_ss(acc, dah, dbh, idesc, (!group_start || ks > 0) ? 1u : 0u);
+              mma_f16_ss(acc, dah, dbl, idesc, 1u);
+              mma_f16_ss(acc, dal, dbh, idesc, 1u);
             }
           }
           mma_commit(&bar_empty[s]);
