@@ -673,7 +673,7 @@ static int pjl_forward(int input_dtype, const void *enc, const void *dec, const 
   if (parts & kPartRest) {
     FRNNT_KERNEL(joiner_band_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(
         logits, stats, symbols, ranges, lse, pxb, pyb, rows, T, R, S, C, blank, L.tiles_n));
-    dim3 grid2((unsigned)((T + 1 + 127) / 128), (unsigned)(S + 1), (unsigned)B);
+    dim3 grid2((unsigned)((T + 1 + 127) / 128), (unsigned)((S + kBandRows) / kBandRows), (unsigned)B);
     FRNNT_KERNEL(band_to_lattice_kernel<float><<<grid2, 128, 0, st>>>(pxb, pyb, ranges, boundary, px, py, S, T, R,
                                                                      rnnt_type, delay_penalty));
     FRNNT_CUDA(cudaGetLastError());

@@ -237,7 +237,7 @@ static int lsm_forward_impl(const void *logits, const int64_t *symbols, const in
 #undef LSM_FWD
 #undef LSM_FWD1
   if (px != nullptr && py != nullptr && B > 0) {
-    dim3 grid2((unsigned)((T + 1 + 127) / 128), (unsigned)(S + 1), (unsigned)B);
+    dim3 grid2((unsigned)((T + 1 + 127) / 128), (unsigned)((S + kBandRows) / kBandRows), (unsigned)B);
     FRNNT_KERNEL(band_to_lattice_kernel<real><<<grid2, 128, 0, st>>>((const real *)pxb, (const real *)pyb,
                                                        ranges, boundary, (real *)px, (real *)py,
                                                        S, T, R, rnnt_type, delay_penalty));

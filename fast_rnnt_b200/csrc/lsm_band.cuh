@@ -46,48 +46,55 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 
 // bands -> lattices: row (ranges[b][t][0] + k) mod (S+1), -inf elsewhere, the -inf column
 // at t = T (regular), the -inf at t = t_end (regular + boundary), px += py[s+1] (constrained),
-// the delay penalty on px
+// the delay penalty on px.  A thread takes one frame of kBandRows lattice rows, so that the
+// frame's shift (a 64-bit load and modulo) is worked out once for all of them: 64 x (100, 500)
+// 20 -> 11 us.
+constexpr int kBandRows = 8;
 template <typename real>
 __global__ void band_to_lattice_kernel(const real *__restrict__ pxb, const real *__restrict__ pyb,
                                        const int64_t *__restrict__ ranges,
                                        const int64_t *__restrict__ boundary, real *__restrict__ px,
                                        real *__restrict__ py, int S, int T, int R, int rnnt_type,
                                        double delay_penalty = 0.0) {
-  const int b = blockIdx.z, s = blockIdx.y;
+  const int b = blockIdx.z, s_first = blockIdx.y * kBandRows;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int S1 = S + 1;
   const int T1 = (rnnt_type == FRNNT_REGULAR) ? T + 1 : T;
   if (t > T) return;
   const real ninf = neg_inf<real>();
-  real vy = ninf, vx = ninf, vy_next = ninf;
-  if (t < T) {
-    const size_t bt = (size_t)b * T + t;
-    long long shift = ranges ? (long long)ranges[bt * R] : 0;
-    shift %= S1;
-    if (shift < 0) shift += S1;
-    int k = s - (int)shift;
-    if (k < 0) k += S1;
-    if (k < R) {
-      vy = pyb[bt * R + k];
-      vx = pxb[bt * R + k];
+  const size_t bt = (size_t)b * T + t;
+  long long shift = ranges && t < T ? (long long)ranges[bt * R] : 0;
+  shift %= S1;
+  if (shift < 0) shift += S1;
+  const bool masked = rnnt_type == FRNNT_REGULAR &&
+                      (t == T || (boundary != nullptr && (long long)t == (long long)boundary[4 * b + 3]));
+  const real penalty = delay_penalty > 0.0 ? delay_penalty_at<real>(boundary, b, T, t, delay_penalty) : (real)0;
+#pragma unroll
+  for (int u = 0; u < kBandRows; ++u) {
+    const int s = s_first + u;
+    if (s > S) break;
+    real vy = ninf, vx = ninf, vy_next = ninf;
+    if (t < T) {
+      int k = s - (int)shift;
+      if (k < 0) k += S1;
+      if (k < R) {
+        vy = pyb[bt * R + k];
+        vx = pxb[bt * R + k];
+      }
+      if (rnnt_type == FRNNT_CONSTRAINED && s < S) {
+        int k1 = s + 1 - (int)shift;
+        if (k1 < 0) k1 += S1;
+        if (k1 >= S1) k1 -= S1;
+        if (k1 < R) vy_next = pyb[bt * R + k1];
+      }
+      py[((size_t)b * S1 + s) * T + t] = vy;
     }
-    if (rnnt_type == FRNNT_CONSTRAINED && s < S) {
-      int k1 = s + 1 - (int)shift;
-      if (k1 < 0) k1 += S1;
-      if (k1 >= S1) k1 -= S1;
-      if (k1 < R) vy_next = pyb[bt * R + k1];
+    if (s < S && t < T1) {
+      if (masked) vx = ninf;
+      if (rnnt_type == FRNNT_CONSTRAINED) vx = vx + vy_next;
+      if (delay_penalty > 0.0) vx = add_rn(vx, penalty);
+      px[((size_t)b * S + s) * T1 + t] = vx;
     }
-    py[((size_t)b * S1 + s) * T + t] = vy;
-  }
-  if (s < S && t < T1) {
-    if (rnnt_type == FRNNT_REGULAR) {
-      if (t == T) vx = ninf;
-      if (boundary != nullptr && (long long)t == (long long)boundary[4 * b + 3]) vx = ninf;
-    } else if (rnnt_type == FRNNT_CONSTRAINED) {
-      vx = vx + vy_next;
-    }
-    if (delay_penalty > 0.0) vx = add_rn(vx, delay_penalty_at<real>(boundary, b, T, t, delay_penalty));
-    px[((size_t)b * S + s) * T1 + t] = vx;
   }
 }
 
