@@ -89,10 +89,10 @@ __device__ __forceinline__ float4 row_load4(const TIn *row, int v, int C) {
                      c + 2 < C ? in_f32(row[c + 2]) : -INFINITY, c + 3 < C ? in_f32(row[c + 3]) : -INFINITY);
 }
 
-// G warps per row of lm (rows 0 .. B*S1-1) or am (the rest), each lane keeping K vectors of four
+// Rows first_row .. rows - 1 of lm (rows 0 .. B*S1-1) and am (the rest), G warps each, each lane keeping K vectors of four
 // entries: a row of up to 128 G K entries is read once.  What bounds the kernel is HBM (read
 // 4 C, write 4 C bytes a row); re-reading what one warp cannot keep made rows of 5000 entries
-// take 1.5 times as long (64 x (60, 400) x 5000: 312 -> 208 us, 157 at the copy rate;
+// take 1.4 times as long (64 x (60, 400) x 5000: 312 -> 226 us, 157 at the copy rate;
 // 16 x (59, 293) x 4233, single entries: 74 -> 40 us).
 template <typename TIn, bool VEC, int G, int K>
 __global__ void __launch_bounds__(256)
@@ -102,12 +102,13 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
                   float *__restrict__ lmmax, float *__restrict__ lmsum, float *__restrict__ ammax,
                   float *__restrict__ lm_blk, float *__restrict__ lm_sym, float *__restrict__ lnorm,
                   float *__restrict__ am_blk, float *__restrict__ am_sym, float *__restrict__ px, int B,
-                  int S, int T, int C, int Cp, int Sp, int blank, int regular) {
+                  int S, int T, int C, int Cp, int Sp, int blank, int regular, long long first_row,
+                  long long rows) {
   constexpr int LANES = 32 * G, RPB = 8 / G;  // threads of a row, rows of a CTA
   __shared__ float part[8];
   const int lane = threadIdx.x % LANES, slot = threadIdx.x / LANES;
   const int S1 = S + 1, nvec = (C + 3) / 4;
-  const long long rows_lm = (long long)B * S1, rows = rows_lm + (long long)B * T;
+  const long long rows_lm = (long long)B * S1;
   auto over_group = [&](float v, bool is_max) {
     v = is_max ? warp_max(v) : warp_sum(v);
     if (G > 1) {
@@ -120,7 +121,7 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
     }
     return v;
   };
-  for (long long row0 = (long long)blockIdx.x * RPB; row0 < rows; row0 += (long long)gridDim.x * RPB) {
+  for (long long row0 = first_row + (long long)blockIdx.x * RPB; row0 < rows; row0 += (long long)gridDim.x * RPB) {
     // a CTA's last rows may not exist; they take part in the barriers of the others
     const bool valid = row0 + slot < rows;
     if (G == 1 && !valid) break;
@@ -428,24 +429,33 @@ __global__ void __launch_bounds__(256)
 sp_split_kernel(const float *__restrict__ x, long long rows, int Tp, int Tq,
                 const float *__restrict__ part, int nparts, __half *__restrict__ hi,
                 __half *__restrict__ lo, float *__restrict__ inv_scale) {
-  __shared__ float slot;
-  if (threadIdx.x < 32) {
-    float m = 0.f;
-    for (int i = threadIdx.x; i < nparts; i += 32) m = fmaxf(m, part[i]);
-    m = warp_max(m);
-    if (threadIdx.x == 0) slot = m;
-  }
+  // the maxima of all rows by all threads of every CTA, four entries at a time after that: read
+  // by one warp, and split entry by entry with a 64-bit division each, 64 x 101 rows of 500
+  // took 19.5 us; 10.8 us this way
+  __shared__ float slot[8];
+  float m = 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < nparts; i += 256) m = fmaxf(m, part[i]);
+  m = warp_max(m);
+  if ((threadIdx.x & 31) == 0) slot[threadIdx.x >> 5] = m;
   __syncthreads();
-  const float scale = fp16_pair_scale(slot);
+#pragma unroll
+  for (int w = 0; w < 8; ++w) m = fmaxf(m, slot[w]);
+  const float scale = fp16_pair_scale(m);
   if (blockIdx.x == 0 && threadIdx.x == 0) *inv_scale = 1.f / scale;
-  const long long n = rows * Tq;
+  const int nvec = Tq / 4;  // Tp is a multiple of 4, too
+  const long long n = rows * nvec;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-    const long long r = i / Tq;
-    const int c = (int)(i - r * Tq);
-    __half h = __float2half_rn(0.f), l = h;
-    if (c < Tp) fp16_pair(x[r * Tp + c], scale, h, l);
-    hi[i] = h;
-    lo[i] = l;
+    const long long r = div_rows(i, nvec);
+    const int c = 4 * (int)(i - r * nvec);
+    uint2 h = make_uint2(0u, 0u), l = h;
+    if (c < Tp) {
+      const float4 q = *reinterpret_cast<const float4 *>(x + r * Tp + c);
+      const float v[4] = {q.x, q.y, q.z, q.w};
+      fp16_pair4(v, scale, h, l);
+    }
+    *reinterpret_cast<uint2 *>(hi + 4 * i) = h;
+    *reinterpret_cast<uint2 *>(lo + 4 * i) = l;
   }
 }
 
@@ -464,27 +474,32 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
   float *am_sym = (float *)(sv + L.am_sym);
   const int S1 = S + 1;
   if (stage == 0) {
-    const long long rows = (long long)B * (S1 + T);
+    const long long rows_lm = (long long)B * S1, rows = rows_lm + (long long)B * T;
     const bool vec = rows_by_four(lm, am, C);
-    // lanes keep 16 entries in rows up to 512, else 32, with as many warps as that takes
-#define FRNNT_EXP_PLANES_AS(TIn, VEC, G, K)                                                                         \
+#define FRNNT_EXP_PLANES_AS(TIn, VEC, G, K, FIRST, LAST)                                                            \
   FRNNT_KERNEL(exp_planes_kernel<TIn, VEC, G, K>                                                                    \
-               <<<(int)std::min<long long>((rows * G + 7) / 8, (long long)sm_count() * 32), 256, 0, st>>>(          \
+               <<<(int)std::min<long long>((((LAST) - (FIRST)) * G + 7) / 8, (long long)sm_count() * 32), 256, 0, st>>>( \
                    (const TIn *)lm, (const TIn *)am, symbols, lp_hi, lp_lo, ap_hi, ap_lo, lmmax, lmsum, ammax,      \
                    lm_blk, lm_sym, lnorm, am_blk, am_sym, px, B, S, T, C, L.Cp, L.Sp, blank,                        \
-                   rnnt_type == FRNNT_REGULAR))
-#define FRNNT_EXP_PLANES_BY(TIn, VEC)       \
-  do {                                      \
-    if (C <= 512)                           \
-      FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 4);  \
-    else if (C <= 1024)                     \
-      FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 8);  \
-    else if (C <= 2048)                     \
-      FRNNT_EXP_PLANES_AS(TIn, VEC, 2, 8);  \
-    else if (C <= 4096)                     \
-      FRNNT_EXP_PLANES_AS(TIn, VEC, 4, 8);  \
-    else                                    \
-      FRNNT_EXP_PLANES_AS(TIn, VEC, 8, 8);  \
+                   rnnt_type == FRNNT_REGULAR, FIRST, LAST))
+    // Rows up to 512: lanes keep 16 entries.  Longer rows: lm, whose sum of exponentials counts,
+    // stays with one warp per row (the order of that sum is kept); am, by far the most rows, goes
+    // to as many warps as 32 entries a lane take
+#define FRNNT_EXP_PLANES_BY(TIn, VEC)                          \
+  do {                                                         \
+    if (C <= 512) {                                            \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 4, 0LL, rows);          \
+    } else {                                                   \
+      FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 4, 0LL, rows_lm);       \
+      if (C <= 1024)                                           \
+        FRNNT_EXP_PLANES_AS(TIn, VEC, 1, 8, rows_lm, rows);    \
+      else if (C <= 2048)                                      \
+        FRNNT_EXP_PLANES_AS(TIn, VEC, 2, 8, rows_lm, rows);    \
+      else if (C <= 4096)                                      \
+        FRNNT_EXP_PLANES_AS(TIn, VEC, 4, 8, rows_lm, rows);    \
+      else                                                     \
+        FRNNT_EXP_PLANES_AS(TIn, VEC, 8, 8, rows_lm, rows);    \
+    }                                                          \
   } while (0)
 #define FRNNT_EXP_PLANES(TIn)            \
   do {                                   \
@@ -553,7 +568,7 @@ int launch_simple_grads_pairs(const float *rw, const float *lmsum, const float *
 
   // the caller left max |rw| per row in `parts`
   const int nparts = (int)rows;
-  const long long nq = rows * Tq;
+  const long long nq = rows * (Tq / 4);
   const int grid = (int)std::min<long long>((nq + 255) / 256, (long long)sm_count() * 16);
   FRNNT_KERNEL(sp_split_kernel<<<grid, 256, 0, st>>>(rw, rows, Tp, Tq, parts, nparts, rw_hi, rw_lo, inv_rw));
   FRNNT_CUDA(cudaGetLastError());
