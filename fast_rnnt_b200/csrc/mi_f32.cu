@@ -6,9 +6,9 @@
 // diagonals) x (time of one step), and everything here shortens the step:
 //
 //   * ONE compute warp per CTA, lane l owning R neighbouring rows: 32 R rows, and a single value
-//     per lane and step travels between threads (a warp shuffle).  R = 1 up to 32 rows, else
-//     2: the second row's instructions fit into the latency of the first row's chain, a third
-//     and fourth would not;
+//     per lane and step travels between threads (a warp shuffle).  R = 1 up to 32 rows (180
+//     cycles a forward step), else 2 (235: the second row's instructions mostly fit into the
+//     latency of the first row's chain; four rows were 2.3 times a step of two);
 //   * a taller lattice is split over a cluster of up to 8 CTAs.  CTA w works two chunks of 16
 //     diagonals behind CTA w - 1 (forward; the other way round in the backward): the compute
 //     warp leaves the edge row in shared memory, an otherwise idle warp sends it, a chunk at
@@ -28,6 +28,9 @@
 //   * the forward's helpers turn the exponents a - p[s][t] that its compute warp leaves in
 //     shared memory into the backward weights (kMiDead: a cell that passes no gradient on), so
 //     that the helpers of the backward only copy them in and the gradients out.
+//
+// Forward / backward of 64 x (100, 500): 79 / 25 us, with one row per thread 113 / 62; of
+// 6 x (423, 2211): 316 / 102 us, before 1240 / 1252.
 #include <cooperative_groups.h>
 
 #include "mi.cuh"
