@@ -102,8 +102,8 @@ def _size_of(device: int, name: str, *args) -> int:
 
 
 def size_of(name: str, *args) -> int:
-    """Result of one of the pure size functions of the C ABI (buffer sizes from tensor sizes; some
-    depend on the current device's number of multiprocessors)."""
+    """Result of one of the size functions of the C ABI: buffer sizes from tensor sizes, some also
+    from the current device's number of multiprocessors, none from an environment switch."""
     return _size_of(torch._C._cuda_getDevice(), name, *args)
 
 

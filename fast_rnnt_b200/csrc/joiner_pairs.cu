@@ -68,9 +68,8 @@ static int launch_pair(const CUtensorMap &mah, const CUtensorMap &mal, const CUt
   return launch_pair_umma<A_MN, B_MN>(mah, mal, mbh, mbl, out, shape, ext, st);
 }
 
-static int pair_tn_splits(int M, int N, long long R) {
+static int pair_tn_splits_for(int tm, int M, int N, long long R) {
   if (M <= 0 || N <= 0 || R <= 0) return 1;
-  const int tm = pair_tile_m(M, true);  // the split products have light epilogues
   const long long tiles = (long long)((M + tm - 1) / tm) * ((N + kPairTile - 1) / kPairTile);
   const long long max_splits = (R + 8 * kPairBK - 1) / (8 * kPairBK);
   const long long sms = sm_count();
@@ -85,6 +84,15 @@ static int pair_tn_splits(int M, int N, long long R) {
     }
   }
   return best;
+}
+static int pair_tn_splits(int M, int N, long long R) {
+  return pair_tn_splits_for(pair_tile_m(M, true), M, N, R);  // the split products have light epilogues
+}
+// the most partial products that a call may leave, whatever FRNNT_PAIR_TILE says by then: buffer
+// sizes do not depend on the switch, so that one asked for (and kept) earlier always suffices
+static int pair_tn_splits_max(int M, int N, long long R) {
+  const int small = pair_tn_splits_for(kPairTile, M, N, R);
+  return M <= kPairTile ? small : std::max(small, pair_tn_splits_for(kP2TileM, M, N, R));
 }
 
 // row groups of the log-softmax backward: each CTA streams a contiguous group of rows for
@@ -152,7 +160,8 @@ static PjlLayout pjl_layout(int B, int T, int R, int S1, int C, int D) {
   L.gz = take(M * D * 4);
   L.rowinfo = take(M * 16);
   L.gmax_part = take(kMaxParts * 4);
-  L.dw_part = take(L.splits > 1 ? (size_t)L.splits * C * D * 4 : 0);
+  const int most = pair_tn_splits_max(C, D, (long long)M);
+  L.dw_part = take(most > 1 ? (size_t)most * C * D * 4 : 0);
   L.cs_part = take((size_t)L.cs_ctas * C * 4);
   L.jg = take(frnnt_joiner_input_grads_scratch_bytes(B, T, D));
   L.bwd_bytes = o;
