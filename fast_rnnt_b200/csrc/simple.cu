@@ -22,6 +22,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "lsm_band.cuh"
 #include "simple_pairs.cuh"
@@ -58,7 +60,7 @@ static inline int rw_pitch(int T) { return (T + 3) & ~3; }
 
 // "scratch": temporaries of one call.
 struct ScratchLayout {
-  size_t rw, sgx, sgy, cgx, cgy, gl, h, partial, dp, rowdot, total;
+  size_t rw, sgx, sgy, cgx, cgy, gl, h, partial, dp, rowdot, weak, weak_row, total;
   int nchunk;
   ScratchLayout(size_t es, int B, int S, int T, int C) {
     size_t o = 0;
@@ -74,6 +76,8 @@ struct ScratchLayout {
     partial = o; o += align_up(es * (size_t)nchunk * C);       // column-sum partials
     dp = o;      o += align_up(es * (size_t)C);                // d loss / d unigram-softmax mean
     rowdot = o;  o += align_up(es * (size_t)B * (S + 1));
+    weak = o;    o += align_up((size_t)B * (S + 1) * weak_words(T) * 4);  // bits of the weak cells
+    weak_row = o; o += align_up((size_t)B * (S + 1));          // lattice row has any
     total = o;
   }
 };
@@ -350,6 +354,341 @@ static int launch_contraction(const Prob &prob, int M, int N, int B, cudaStream_
   return FRNNT_OK;
 }
 
+// ---- weak cells (simple_pairs.cuh): float32 products where the planes do not hold ---------------------
+// acc[m][n] = sum_k X(m,k) Y(n,k) of one 64 x 64 tile, 16 entries per thread.  What bounds it is the
+// latency of its loads (few tiles, long reductions): the operands of the next 16 k are
+// fetched into registers while this slice's products run, and two buffers in shared memory leave
+// one barrier per slice.  An operand says how a thread's four values of a slice are fetched and
+// where (and through which function) they are placed.
+constexpr int kWeakTile = 64, kWeakBK = 16, kWeakThreads = 256, kWeakPitch = kWeakTile + 4;
+typedef float WeakSlice[kWeakBK][kWeakPitch];
+
+template <class X, class Y>
+__device__ __forceinline__ void weak_product(X &x, Y &y, int K, WeakSlice (&Xs)[2], WeakSlice (&Ys)[2],
+                                             float (&acc)[4][4]) {
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  float xv[4], yv[4];
+  x.fetch(0, K, xv);
+  y.fetch(0, K, yv);
+  for (int k0 = 0, buf = 0; k0 < K; k0 += kWeakBK, buf ^= 1) {
+    x.place(k0, xv, Xs[buf]);
+    y.place(k0, yv, Ys[buf]);
+    __syncthreads();
+    if (k0 + kWeakBK < K) {
+      x.fetch(k0 + kWeakBK, K, xv);
+      y.fetch(k0 + kWeakBK, K, yv);
+    }
+#pragma unroll
+    for (int k = 0; k < kWeakBK; ++k) {
+      const float4 a = *reinterpret_cast<const float4 *>(&Xs[buf][k][4 * ty]);
+      const float4 b = *reinterpret_cast<const float4 *>(&Ys[buf][k][4 * tx]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * bv[j];
+    }
+  }
+  __syncthreads();  // the buffers are free again
+}
+
+// e^{row - max} of 64 rows, k along the row: thread <-> (row tid / 16 + 16 e, k tid % 16)
+template <typename TIn>
+struct WeakRows {
+  const TIn *row[4];  // nullptr: no such row
+  float mx[4];
+  __device__ void fetch(int k0, int K, float (&v)[4]) const {
+    const int k = k0 + threadIdx.x % 16;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = row[e] != nullptr && k < K ? in_f32(row[e][k]) : -INFINITY;
+  }
+  __device__ void place(int, const float (&v)[4], WeakSlice &s) const {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[threadIdx.x % 16][threadIdx.x / 16 + 16 * e] = expf(v[e] - mx[e]);
+  }
+};
+
+// A CTA takes 64 lattice rows (constrained: 63, and the one that px of the last needs) and the
+// blockIdx.x-th 64 of the frames that have weak cells among them; it leaves at once where there
+// are none.  All its cells go through the product, the weak ones are replaced, and py and px
+// follow from the normalizers.  64 x (100, 500) x 500: 4 us with nothing weak, 211 us with every
+// cell weak; 16 x (59, 293) x 4233: 2 and 273 us.
+template <typename TIn>
+__global__ void __launch_bounds__(kWeakThreads)
+weak_cells_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am, SimpleLattice q) {
+  __shared__ __align__(16) WeakSlice Xs[2], Ys[2];
+  __shared__ int frames[kWeakTile], counts[8];
+  __shared__ uint8_t replaced[kWeakTile][16];  // bits of four rows each, per frame
+  const int tid = threadIdx.x, lane = tid & 31, b = blockIdx.z;
+  const bool constrained = q.rnnt_type == FRNNT_CONSTRAINED;
+  const int s0 = blockIdx.y * (constrained ? kWeakTile - 1 : kWeakTile);
+  const int S1 = q.S + 1, T = q.T, C = q.C;
+  // flags per 128 rows; constrained lattices have one such tile
+  const uint8_t *weak = q.weak + ((size_t)b * ((S1 + 127) / 128) + (constrained ? 0 : s0 / 128)) * T;
+  bool any = false;
+  for (int t = tid; t < T; t += kWeakThreads) any |= weak[t];
+  if (!__syncthreads_or(any)) return;
+  const int first = blockIdx.x * kWeakTile;
+  int found = 0;
+  for (int t0 = 0; t0 < T; t0 += kWeakThreads) {
+    const int t = t0 + tid;
+    const bool w = t < T && weak[t];
+    const unsigned m = __ballot_sync(0xffffffffu, w);
+    if (lane == 0) counts[tid >> 5] = __popc(m);
+    __syncthreads();
+    int at = found - first + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i < tid >> 5) at += counts[i];
+      found += counts[i];
+    }
+    if (w && at >= 0 && at < kWeakTile) frames[at] = t;
+    __syncthreads();
+  }
+  const int nframes = min(kWeakTile, found - first), rows = min(kWeakTile, S1 - s0);
+  if (nframes <= 0) return;
+  const size_t bs0 = (size_t)b * S1 + s0, bt0 = (size_t)b * T;
+  WeakRows<TIn> x, y;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int m = tid / 16 + 16 * e;
+    x.row[e] = m < rows ? lm + (bs0 + m) * C : nullptr;
+    x.mx[e] = m < rows ? q.lmmax[bs0 + m] : 0.f;
+    y.row[e] = m < nframes ? am + (bt0 + frames[m]) * C : nullptr;
+    y.mx[e] = m < nframes ? q.ammax[bt0 + frames[m]] : 0.f;
+  }
+  float acc[4][4] = {};
+  weak_product(x, y, C, Xs, Ys, acc);
+  const int tx = tid % 16, ty = tid / 16;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int n = 4 * tx + j;
+    if (n >= nframes) break;
+    const size_t bt = bt0 + frames[n];
+    const float ax = q.ammax[bt], asum = q.am_sum[bt];
+    unsigned bits = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int s = 4 * ty + i;
+      if (s >= rows || !(acc[i][j] < weak_bound(q.lmsum[bs0 + s], asum))) continue;
+      bits |= 1u << i;
+      q.norm[(bs0 + s) * T + frames[n]] = logf(acc[i][j] + 1.17549435e-38f) + q.lmmax[bs0 + s] + ax;
+    }
+    replaced[n][ty] = (uint8_t)bits;
+  }
+  __syncthreads();
+  const int T1 = q.rnnt_type == FRNNT_REGULAR ? T + 1 : T;
+  const bool am_on = q.smoothed && !q.am_only_off;
+  for (int idx = tid; idx < nframes * kWeakTile; idx += kWeakThreads) {
+    const int n = idx / kWeakTile, t = frames[n], i = idx % kWeakTile, s = s0 + i;
+    const bool here = replaced[n][i / 4] >> (i % 4) & 1;
+    const bool next = constrained && i + 1 < kWeakTile && (replaced[n][(i + 1) / 4] >> ((i + 1) % 4) & 1);
+    if (!here && !next) continue;
+    const size_t bt = bt0 + t;
+    auto py_of = [&](int k) {
+      const size_t bs = bs0 + k;
+      float v = q.am_blk[bt] + q.lm_blk[bs] - q.norm[bs * T + t];
+      if (q.smoothed) v = v * q.both + (q.lm_blk[bs] - q.lnorm[bs]) * q.ls;
+      if (am_on) v += (q.am_blk[bt] + q.loguni[q.blank] - q.amonly[bt]) * q.as;
+      return v;
+    };
+    if (here) q.py[(bs0 + i) * T + t] = py_of(i);
+    if (s >= q.S || (constrained && i == kWeakTile - 1)) continue;  // (that row is the next CTA's first)
+    const size_t bs = bs0 + i;
+    const float px_am = q.am_sym[bt * q.Sp + s], px_lm = q.lm_sym[bs];
+    float v = px_am + px_lm - q.norm[bs * T + t];
+    if (q.smoothed) v = v * q.both + (px_lm - q.lnorm[bs]) * q.ls;
+    if (am_on) {
+      long long c = q.symbols[(size_t)b * q.S + s];
+      if (c < 0 || c >= C) c = q.blank;
+      v += (px_am + q.loguni[c] - q.amonly[bt]) * q.as;
+    }
+    if (q.rnnt_type == FRNNT_REGULAR) {
+      if (q.boundary != nullptr && (long long)t == (long long)q.boundary[4 * b + 3]) v = -INFINITY;
+    } else if (constrained) {
+      v += py_of(i + 1);
+    }
+    if (q.delay_penalty > 0.0) v = add_rn(v, delay_penalty_at<float>(q.boundary, b, T, t, q.delay_penalty));
+    q.px[((size_t)b * q.S + s) * T1 + t] = v;
+  }
+}
+
+// calls f with lm and am as pointers to their type
+template <class F>
+static void with_input_type(int input_dtype, const void *lm, const void *am, F f) {
+  if (input_dtype == FRNNT_F16)
+    f((const __half *)lm, (const __half *)am);
+  else if (input_dtype == FRNNT_BF16)
+    f((const __nv_bfloat16 *)lm, (const __nv_bfloat16 *)am);
+  else
+    f((const float *)lm, (const float *)am);
+}
+
+int launch_weak_cells(const void *lm, const void *am, int input_dtype, const SimpleLattice &lattice, int B,
+                      cudaStream_t st) {
+  const int step = lattice.rnnt_type == FRNNT_CONSTRAINED ? kWeakTile - 1 : kWeakTile;
+  const dim3 grid((unsigned)((lattice.T + kWeakTile - 1) / kWeakTile), (unsigned)((lattice.S + step) / step),
+                  (unsigned)B);
+  with_input_type(input_dtype, lm, am, [&](auto *l, auto *a) {
+    FRNNT_KERNEL(weak_cells_kernel<<<grid, kWeakThreads, 0, st>>>(l, a, lattice));
+  });
+  FRNNT_CUDA(cudaGetLastError());
+  return FRNNT_OK;
+}
+
+// What weak cells add to the gradients, dlm[s][c] -= L[s][c] sum_t Rw[s][t] A[t][c] and
+// dam[t][c] -= A[t][c] sum_s Rw[s][t] L[s][c] over the weak cells, and the am-only term of frames
+// whose am-only normalizer is weak.
+template <typename TIn>
+struct WeakGrads {
+  const TIn *lm, *am;
+  const float *rw;
+  const unsigned *weak;      // bits of the weak cells, [B][S1][words]
+  const uint8_t *weak_row;   // [B][S1]
+  const float *lmmax, *ammax, *amonly, *h, *uni;
+  float *lm_grad, *am_grad;
+  int B, S1, T, C, Tp;
+};
+// Rw of the weak cells of 64 rows of lm or am, k through a list of frames resp. lattice rows;
+// neighbouring threads on neighbouring frames either way
+struct WeakWeights {
+  const float *rw;
+  const unsigned *weak;
+  const int *list;
+  bool is_lm;
+  int m0, M, Tp, words;
+  unsigned word[4];
+  int bit[4];
+  __device__ int k_of(int e) const { return is_lm ? threadIdx.x % 16 : threadIdx.x / 64 + 4 * e; }
+  __device__ int m_of(int e) const { return is_lm ? threadIdx.x / 16 + 16 * e : threadIdx.x % 64; }
+  // the weight and the word that says whether it counts: neither load waits for the other
+  __device__ void fetch(int k0, int K, float (&v)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = k0 + k_of(e), m = m0 + m_of(e);
+      v[e] = 0.f, word[e] = 0u, bit[e] = 0;
+      if (k >= K || m >= M) continue;
+      const int at = list[k], s = is_lm ? m : at, t = is_lm ? at : m;
+      word[e] = weak[(size_t)s * words + t / 32];
+      bit[e] = t % 32;
+      v[e] = rw[(size_t)s * Tp + t];
+    }
+  }
+  __device__ void place(int, const float (&v)[4], WeakSlice &s) const {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[k_of(e)][m_of(e)] = word[e] >> bit[e] & 1u ? v[e] : 0.f;
+  }
+};
+// e^{row - max}, rows through the list, 64 columns: thread <-> (column tid % 64, k tid / 64 + 4 e)
+template <typename TIn>
+struct WeakColumns {
+  const TIn *x;
+  const float *mx;
+  const int *list;
+  int n0, C;
+  float m[4];
+  __device__ void fetch(int k0, int K, float (&v)[4]) {
+    const int c = n0 + threadIdx.x % 64;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = k0 + threadIdx.x / 64 + 4 * e;
+      const bool ok = k < K && c < C;
+      v[e] = ok ? in_f32(x[(size_t)list[k] * C + c]) : -INFINITY;
+      m[e] = ok ? mx[list[k]] : 0.f;
+    }
+  }
+  __device__ void place(int, const float (&v)[4], WeakSlice &s) const {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[threadIdx.x / 64 + 4 * e][threadIdx.x % 64] = expf(v[e] - m[e]);
+  }
+};
+
+// A CTA takes 64 rows of lm (of am) and every lm_split-th (am_split-th) 64 columns; it leaves at once
+// when the rows have nothing weak.  The frames (lattice rows) that some of its rows need are
+// listed, kWeakList candidates at a time, and the product runs over the list.  64 x (100, 500) x
+// 500: 4.5 us with nothing weak, 507 us with every cell weak (the whole gradient 750 us then; the
+// FMA pipe for every cell 660); 16 x (59, 293) x 4233: 4.7 and 450 us (670; 660).  128 x 128 tiles
+// without prefetch, as the FMA pipe's, took two to seven times as long for either kernel.
+constexpr int kWeakList = 1024;
+template <typename TIn>
+__global__ void __launch_bounds__(kWeakThreads, 3)
+weak_grads_kernel(const WeakGrads<TIn> g, int lm_split, int am_split) {
+  __shared__ __align__(16) WeakSlice Xs[2], Ys[2];
+  __shared__ int list[kWeakList], counts[8];
+  const int tid = threadIdx.x, lane = tid & 31, tx = tid % 16, ty = tid / 16;
+  const int words = weak_words(g.T);
+  const int lm_tiles = (g.S1 + kWeakTile - 1) / kWeakTile, am_tiles = (g.T + kWeakTile - 1) / kWeakTile;
+  const long long lm_ctas = (long long)g.B * lm_tiles * lm_split;
+  const bool is_lm = blockIdx.x < lm_ctas;
+  const int split = is_lm ? lm_split : am_split, tiles = is_lm ? lm_tiles : am_tiles;
+  const int cta = (int)(is_lm ? blockIdx.x : blockIdx.x - lm_ctas), item = cta / split;
+  const int b = item / tiles, m0 = kWeakTile * (item % tiles);
+  const int M = is_lm ? g.S1 : g.T, depth = is_lm ? g.T : g.S1;
+  const size_t lm0 = (size_t)b * g.S1, am0 = (size_t)b * g.T;
+  bool cells = false, frames = false;
+  const int end = is_lm ? min(m0 + kWeakTile, g.S1) : g.S1;
+  for (int s = (is_lm ? m0 : 0) + tid; s < end; s += kWeakThreads) cells |= g.weak_row[lm0 + s];
+  if (!is_lm && g.h != nullptr && tid < kWeakTile && m0 + tid < g.T)
+    frames = am_only_weak(g.ammax[am0 + m0 + tid], g.amonly[am0 + m0 + tid]);
+  cells = __syncthreads_or(cells);
+  frames = __syncthreads_or(frames);
+  if (!cells && !frames) return;
+  const unsigned *weak = g.weak + lm0 * words;
+  const float *rw = g.rw + lm0 * g.Tp;
+  for (int n0 = (cta % split) * kWeakTile; n0 < g.C; n0 += split * kWeakTile) {
+    float acc[4][4] = {};
+    for (int d0 = 0; cells && d0 < depth; d0 += kWeakList) {
+      int K = 0;
+      for (int k0 = d0; k0 < min(depth, d0 + kWeakList); k0 += kWeakThreads) {
+        const int k = k0 + tid;
+        unsigned used = 0;
+        if (k < depth) {
+          if (is_lm) {
+            for (int s = m0; s < end; ++s) used |= weak[(size_t)s * words + k / 32] >> (k % 32) & 1u;
+          } else {
+            used = weak[(size_t)k * words + m0 / 32];
+            if (m0 / 32 + 1 < words) used |= weak[(size_t)k * words + m0 / 32 + 1];
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, used != 0);
+        if (lane == 0) counts[tid >> 5] = __popc(m);
+        __syncthreads();
+        int at = K + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i < tid >> 5) at += counts[i];
+          K += counts[i];
+        }
+        if (used != 0) list[at] = k;
+        __syncthreads();
+      }
+      WeakColumns<TIn> y{is_lm ? g.am + am0 * g.C : g.lm + lm0 * g.C, is_lm ? g.ammax + am0 : g.lmmax + lm0, list, n0,
+                         g.C, {}};
+      WeakWeights x{rw, weak, list, is_lm, m0, M, g.Tp, words, {}, {}};
+      weak_product(x, y, K, Xs, Ys, acc);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + 4 * ty + i;
+      if (m >= M) break;
+      const size_t row = (is_lm ? lm0 : am0) + m;
+      const float own_max = is_lm ? g.lmmax[row] : g.ammax[row];
+      const TIn *own = (is_lm ? g.lm : g.am) + row * g.C;
+      float *grad = (is_lm ? g.lm_grad : g.am_grad) + row * g.C;
+      // the am-only term of a weak frame: h u[c] / Z
+      const float frame = frames && am_only_weak(own_max, g.amonly[row]) ? g.h[row] * expf(own_max - g.amonly[row]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = n0 + 4 * tx + j;
+        if (c >= g.C) break;
+        float v = acc[i][j];
+        if (frame != 0.f) v += frame * g.uni[c];
+        if (v != 0.f) grad[c] -= expf(in_f32(own[c]) - own_max) * v;
+      }
+    }
+  }
+}
+
 // ---- lattice assembly -------------------------------------------------------------
 struct SmoothCfg {
   int smoothed;
@@ -473,39 +812,56 @@ __global__ void grad_weight_kernel(EffGrads<real> eg, const real *__restrict__ n
 
 // The two kernels above and below in one pass, for the tensor-core path: one CTA per lattice
 // row (b, s) writes the row of Rw, the row sums of gx (all T1 columns) and gy, and the
-// row's largest |Rw| (which sets the scale of the fp16 planes Rw is split into).
+// row's largest |Rw| (which sets the scale of the fp16 planes Rw is split into).  Weak cells
+// (simple_pairs.cuh) do not go into the planes: their bits go to `weak`, weak_row says whether
+// the row has any.
 template <typename real>
 __global__ void __launch_bounds__(128)
 grad_weight_rows_kernel(EffGrads<real> eg, const real *__restrict__ norm, const real *__restrict__ lmmax,
-                        const real *__restrict__ ammax, real *__restrict__ rw, real *__restrict__ sgx,
-                        real *__restrict__ sgy, float *__restrict__ rowmax, real both, int Tp) {
+                        const real *__restrict__ ammax, const real *__restrict__ lmsum,
+                        const float *__restrict__ am_sum, real *__restrict__ rw, real *__restrict__ sgx,
+                        real *__restrict__ sgy, float *__restrict__ rowmax, unsigned *__restrict__ weak,
+                        uint8_t *__restrict__ weak_row, real both, int Tp) {
   __shared__ real red[3][4];
   const int row = blockIdx.x, b = row / (eg.S + 1), s = row % (eg.S + 1);
   const real lmx = lmmax[row];
+  const float lms = (float)lmsum[row];
+  const int words = weak_words(eg.T);
+  bool any_weak = false;
   real ax = 0, ay = 0, mx = 0;
   const int n = max(Tp, eg.T1);
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    const real gx = eg.gx(b, s, t), gy = eg.gy(b, s, t);
-    ax += gx;
-    ay += gy;
-    if (t < Tp) {
-      real v = 0;
-      if (t < eg.T) {
-        const real w = both * (gx + gy);
-        const real inv = exp_r(lmx + ammax[(size_t)b * eg.T + t] - norm[(size_t)row * eg.T + t]);
-        v = (w == 0) ? (real)0 : w * inv;
+  for (int t0 = 0; t0 < n; t0 += 128) {
+    const int t = t0 + threadIdx.x;
+    bool is_weak = false;
+    if (t < n) {
+      const real gx = eg.gx(b, s, t), gy = eg.gy(b, s, t);
+      ax += gx;
+      ay += gy;
+      if (t < Tp) {
+        real v = 0;
+        if (t < eg.T) {
+          const real w = both * (gx + gy);
+          const real inv = exp_r(lmx + ammax[(size_t)b * eg.T + t] - norm[(size_t)row * eg.T + t]);
+          v = (w == 0) ? (real)0 : w * inv;
+          // 1 / z against the bound; a cell without weight counts nowhere
+          is_weak = w != 0 && (float)inv * weak_bound(lms, am_sum[(size_t)b * eg.T + t]) > 1.f;
+        }
+        rw[(size_t)row * Tp + t] = v;
+        if (!is_weak) mx = max(mx, v < 0 ? -v : v);
       }
-      rw[(size_t)row * Tp + t] = v;
-      mx = max(mx, v < 0 ? -v : v);
     }
+    const unsigned bits = __ballot_sync(0xffffffffu, is_weak);
+    if ((threadIdx.x & 31) == 0 && t / 32 < words) weak[(size_t)row * words + t / 32] = bits;
+    any_weak |= is_weak;
   }
   ax = warp_sum(ax);
   ay = warp_sum(ay);
   mx = warp_max(mx);
   const int w = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) red[0][w] = ax, red[1][w] = ay, red[2][w] = mx;
-  __syncthreads();
+  any_weak = __syncthreads_or(any_weak);
   if (threadIdx.x == 0) {
+    weak_row[row] = any_weak;
     sgx[row] = (red[0][0] + red[0][1]) + (red[0][2] + red[0][3]);
     sgy[row] = (red[1][0] + red[1][1]) + (red[1][2] + red[1][3]);
     rowmax[row] = (float)max(max(red[2][0], red[2][1]), max(red[2][2], red[2][3]));
@@ -686,6 +1042,33 @@ __global__ void row_dot_kernel(const real *__restrict__ lm, const real *__restri
   if (lane == 0) rowdot[row] = acc / lmsum[row];
 }
 
+// The same sum and what it stands for, lm_grad[row][c] += P[row][c] (dP[c] - rowdot[row]), for the
+// tensor-core path: one CTA per lm row, which the second pass finds in the caches.  P in
+// float32: dP[c] goes up to 1 / (rows u[c]) for a symbol that is improbable in every row, where
+// the planes would lose P.
+__global__ void __launch_bounds__(256)
+lm_unigram_grad_kernel(const float *__restrict__ lm, const float *__restrict__ lmmax,
+                       const float *__restrict__ lmsum, const float *__restrict__ dp,
+                       float *__restrict__ lm_grad, int C) {
+  __shared__ float part[8];
+  const long long row = blockIdx.x;
+  const float *src = lm + row * C;
+  float *dst = lm_grad + row * C;
+  const float m = lmmax[row], sum = lmsum[row];
+  float acc = 0.f;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < C; c += 256) acc += expf(src[c] - m) * dp[c];
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  acc = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) acc += part[w];
+  const float rowdot = acc / sum;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < C; c += 256) dst[c] += expf(src[c] - m) / sum * (dp[c] - rowdot);
+}
+
 // tensor-core (tcgen05, 3xTF32) contraction, FRNNT_CONTRACTION=tf32 or tall constrained lattices:
 // float32 with 16-byte aligned rows; what else the fp16-pair engine does not take (float64,
 // tall constrained lattices with an odd vocabulary) runs on the SIMT path.  The
@@ -799,7 +1182,8 @@ static int simple_forward_impl(const void *lm_, const void *am_, const int64_t *
                                        rnnt_type, cfg.smoothed, cfg.am_only_off, (float)cfg.both,
                                        (float)cfg.ls, (float)cfg.as, (float *)px, (float *)py, (float *)norm,
                                        (float *)lmmax, (float *)lmsum, (float *)ammax, (const float *)amonly,
-                                       (const float *)loguni, pairs_saved, B, S, T, C, 1, st, cfg.delay_penalty);
+                                       (const float *)loguni, pairs_saved, B, S, T, C, 1, st, cfg.delay_penalty,
+                                       input_dtype);
   if (use_tensor_cores<real>(lm, am, S1, T, C)) {
     rc = launch_norm_umma((const float *)lm, (const float *)am, (const float *)lmmax,
                           (const float *)ammax, (float *)norm, B, S1, T, C, st);
@@ -821,8 +1205,8 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
                                 const int64_t *boundary, int blank, int rnnt_type, SmoothCfg cfg,
                                 int am_only_active, const void *px_grad, const void *py_grad,
                                 const void *saved, void *scratch, void *lm_grad_, void *am_grad_,
-                                int B, int S, int T, int C, cudaStream_t st) {
-  const real *lm = (const real *)lm_, *am = (const real *)am_;
+                                int B, int S, int T, int C, cudaStream_t st, int input_dtype) {
+  const real *lm = (const real *)lm_, *am = (const real *)am_;  // 16-bit inputs: only weak_grads_kernel reads them
   real *lm_grad = (real *)lm_grad_, *am_grad = (real *)am_grad_;
   const int S1 = S + 1;
   const int T1 = rnnt_type == FRNNT_REGULAR ? T + 1 : T;
@@ -844,11 +1228,14 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
   const int Tp = rw_pitch(T);
   const bool pairs = use_pairs<real>(lm, am, S1, T, C, rnnt_type) && T > 0;
   dim3 g3((unsigned)((Tp + 127) / 128), (unsigned)S1, (unsigned)B);
+  const float *am_sum = (const float *)(svb + sv.total + simple_pairs_amsum_offset(B, S, T, C));
+  unsigned *weak = (unsigned *)(scb + sc.weak);
+  uint8_t *weak_row = (uint8_t *)(scb + sc.weak_row);
   if (pairs) {
     // one pass: Rw, the row sums and the row maxima of |Rw| (first floats of the pairs scratch)
     FRNNT_KERNEL(grad_weight_rows_kernel<real><<<(unsigned)lm_rows, 128, 0, st>>>(
-        eg, norm, lmmax, ammax, rw, sgx, sgy, (float *)(scb + sc.total + simple_pairs_rowmax_offset(B, S, T, C)),
-        (real)cfg.both, Tp));
+        eg, norm, lmmax, ammax, lmsum, am_sum, rw, sgx, sgy,
+        (float *)(scb + sc.total + simple_pairs_rowmax_offset(B, S, T, C)), weak, weak_row, (real)cfg.both, Tp));
   } else {
     if (T > 0)
       FRNNT_KERNEL(grad_weight_kernel<real><<<g3, 128, 0, st>>>(eg, norm, lmmax, ammax, rw, (real)cfg.both, Tp));
@@ -874,8 +1261,9 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
       FRNNT_KERNEL(column_partial_kernel<real, 1><<<g1, 128, 0, st>>>(am, ammax, amonly, h, partial, am_rows, C));
       FRNNT_KERNEL(unigram_grad_kernel<real><<<(C + kUniRows - 1) / kUniRows, kUniRows, 0, st>>>(symbols, sgx, sgy, partial, nchunk,
                                                             uni, dp, B, S, C, blank, (real)cfg.as));
-      FRNNT_KERNEL(row_dot_kernel<real><<<(int)((lm_rows * 32 + 255) / 256), 256, 0, st>>>(lm, lmmax, lmsum, dp,
-                                                                         rowdot, lm_rows, C));
+      if (!pairs)
+        FRNNT_KERNEL(row_dot_kernel<real><<<(int)((lm_rows * 32 + 255) / 256), 256, 0, st>>>(lm, lmmax, lmsum, dp,
+                                                                           rowdot, lm_rows, C));
       dp_p = dp;
       rowdot_p = rowdot;
     }
@@ -884,12 +1272,30 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
 
   int rc;
   if (pairs) {
-    rc = launch_simple_grads_pairs((const float *)rw, (const float *)lmsum, (const float *)ammax,
+    rc = launch_simple_grads_pairs((const float *)rw, weak, (const float *)lmsum, (const float *)ammax,
                                    (const float *)amonly, (const float *)uni, (const float *)gl_p,
-                                   (const float *)h_p, (const float *)dp_p, (const float *)rowdot_p,
-                                   (float *)lm_grad, (float *)am_grad, svb + sv.total, scb + sc.total, B, S, T,
-                                   C, Tp, st);
+                                   (const float *)h_p, (float *)lm_grad, (float *)am_grad, svb + sv.total,
+                                   scb + sc.total, B, S, T, C, Tp, st);
     if (rc != FRNNT_OK) return rc;
+    if (dp_p != nullptr)
+      FRNNT_KERNEL(lm_unigram_grad_kernel<<<(unsigned)lm_rows, 256, 0, st>>>(
+          (const float *)lm, (const float *)lmmax, (const float *)lmsum, (const float *)dp_p, (float *)lm_grad, C));
+    // four CTAs per SM for either side, where there are as many: a tile's columns over several
+    // (eight: 6% faster where everything is weak, 7 instead of 4.5 us where nothing is)
+    const long long tiles_c = (C + kWeakTile - 1) / kWeakTile, most = (long long)sm_count() * 4;
+    const long long lm_items = (long long)B * ((S1 + kWeakTile - 1) / kWeakTile);
+    const long long am_items = (long long)B * ((T + kWeakTile - 1) / kWeakTile);
+    const int lm_split = (int)std::min(tiles_c, std::max(1LL, most / lm_items));
+    const int am_split = (int)std::min(tiles_c, std::max(1LL, most / am_items));
+    const unsigned ctas = (unsigned)(lm_items * lm_split + am_items * am_split);
+    with_input_type(input_dtype, lm_, am_, [&](auto *l, auto *a) {
+      using TIn = std::remove_const_t<std::remove_pointer_t<decltype(l)>>;
+      const WeakGrads<TIn> g{l, a, (const float *)rw, weak, weak_row, (const float *)lmmax, (const float *)ammax,
+                             (const float *)amonly, (const float *)h_p, (const float *)uni, (float *)lm_grad,
+                             (float *)am_grad, B, S1, T, C, Tp};
+      FRNNT_KERNEL(weak_grads_kernel<<<ctas, kWeakThreads, 0, st>>>(g, lm_split, am_split));
+    });
+    FRNNT_CUDA(cudaGetLastError());
   } else if (use_tensor_cores<real>(lm, am, S1, T, C)) {
     rc = launch_simple_grads_umma((const float *)lm, (const float *)am, (const float *)lmmax,
                                   (const float *)lmsum, (const float *)ammax, (const float *)amonly,
@@ -985,15 +1391,14 @@ extern "C" int frnnt_simple_logprobs_backward(int dtype, const void *lm, const v
   const int am_only_active = smoothed && am_only_scale != 0.0;
   cudaStream_t st = (cudaStream_t)stream;
   if (is_half_input(dtype)) {
-    // lm and am are not read on this path (the forward kept what the backward needs)
     FRNNT_REQUIRE(use_pairs<float>(lm, am, S + 1, T, C, rnnt_type) && T > 0 && !am_only_active,
                   FRNNT_EUNSUPPORTED, "16-bit inputs: see frnnt_simple_reads_16bit_inputs");
   }
   if (dtype != FRNNT_F64)
     return simple_backward_impl<float>(lm, am, symbols, boundary, blank, rnnt_type, cfg,
                                        am_only_active, px_grad, py_grad, saved, scratch, lm_grad,
-                                       am_grad, B, S, T, C, st);
+                                       am_grad, B, S, T, C, st, dtype);
   return simple_backward_impl<double>(lm, am, symbols, boundary, blank, rnnt_type, cfg,
                                       am_only_active, px_grad, py_grad, saved, scratch, lm_grad,
-                                      am_grad, B, S, T, C, st);
+                                      am_grad, B, S, T, C, st, dtype);
 }

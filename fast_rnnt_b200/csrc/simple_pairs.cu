@@ -14,7 +14,8 @@
 //   backward  the gradient weights Rw[s][t] (simple.cu) become planes, and
 //             dlm[s][c] = -L[s][c] * sum_t Rw[s][t] A[t][c],
 //             dam[t][c] = -A[t][c] * sum_s Rw[s][t] L[s][c]
-//             run on the same engine, L and A read back from the planes in the epilogue.
+//             run on the same engine, L and A read back from the planes in the epilogue;
+//   weak cells (simple_pairs.cuh) are computed in float32, forward and backward.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -51,6 +52,8 @@ SimplePairsLayout::SimplePairsLayout(int B, int S, int T, int C) {
   lnorm = take((size_t)B * S1 * 4);
   am_blk = take((size_t)B * T * 4);
   am_sym = take((size_t)B * T * Sp * 4);
+  am_sum = take((size_t)B * T * 4);
+  weak = take((size_t)B * ((S1 + kPairTile - 1) / kPairTile) * T);
   saved_bytes = o;
   o = 0;
   rw_hi = take((size_t)B * S1 * Tq * 2);
@@ -61,6 +64,7 @@ SimplePairsLayout::SimplePairsLayout(int B, int S, int T, int C) {
 }
 
 size_t simple_pairs_rowmax_offset(int B, int S, int T, int C) { return SimplePairsLayout(B, S, T, C).parts; }
+size_t simple_pairs_amsum_offset(int B, int S, int T, int C) { return SimplePairsLayout(B, S, T, C).am_sum; }
 
 bool simple_pairs_supported(const void *lm, const void *am, int S1, int T, int C, int rnnt_type) {
   (void)lm, (void)am;  // rows of any alignment: see rows_by_four
@@ -101,8 +105,8 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
                   __half *__restrict__ lp_lo, __half *__restrict__ ap_hi, __half *__restrict__ ap_lo,
                   float *__restrict__ lmmax, float *__restrict__ lmsum, float *__restrict__ ammax,
                   float *__restrict__ lm_blk, float *__restrict__ lm_sym, float *__restrict__ lnorm,
-                  float *__restrict__ am_blk, float *__restrict__ am_sym, float *__restrict__ px, int B,
-                  int S, int T, int C, int Cp, int Sp, int blank, int regular, long long first_row,
+                  float *__restrict__ am_blk, float *__restrict__ am_sym, float *__restrict__ am_sum,
+                  float *__restrict__ px, int B, int S, int T, int C, int Cp, int Sp, int blank, int regular, long long first_row,
                   long long rows) {
   constexpr int LANES = 32 * G, RPB = 8 / G;  // threads of a row, rows of a CTA
   __shared__ float part[8];
@@ -196,6 +200,7 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
         }
       } else {
         ammax[r] = m;
+        am_sum[r] = sum;
         am_blk[r] = in_f32(x[blank]);
       }
     }
@@ -208,22 +213,14 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
 // vocabularies that the FMA pipe used to serve, whose float32 sums were more accurate than 128
 // truncating tensor-core additions (C = 50 .. 500: relative error of px 1.0e-7 against 5.5e-8)
 template <bool EXACT>
-struct NormPairExt {
+struct NormPairExt : SimpleLattice {
   static constexpr bool kBatched = true, kCustomStore = true;
   static constexpr int kGroup = EXACT ? 1 : kPairGroup;
-  float *norm, *px, *py;
-  const float *am_sym;  // [B][T][Sp]
-  const int64_t *symbols, *boundary;
-  const float *lmmax, *ammax, *lm_blk, *lm_sym, *lnorm, *am_blk, *amonly, *loguni;
-  int S, T, C, blank, rnnt_type;
-  int smoothed, am_only_off;
-  float both, ls, as;
-  int Sp;
-  double delay_penalty;
   struct Row {
-    float ammax_t, am_blk_t, amonly_t, py_next, pen;
+    float ammax_t, am_blk_t, amonly_t, py_next, pen, am_sum_t;
     const float *amrow;
     long long t_end;
+    bool weak;
   };
   __device__ void row_begin(Row &r, int b, int t, int) const {
     const size_t bt = (size_t)b * T + t;
@@ -234,15 +231,21 @@ struct NormPairExt {
     r.t_end = (rnnt_type == FRNNT_REGULAR && boundary != nullptr) ? (long long)boundary[4 * b + 3] : -1;
     r.py_next = 0.f;
     r.pen = delay_penalty_at<float>(boundary, b, T, t, delay_penalty);
+    r.am_sum_t = am_sum[bt];
+    r.weak = false;
   }
   __device__ void prefetch(Row &, int, int, int) const {}
   __device__ void finish(Row &, int, int, int, float (&)[16], int) const {}
-  __device__ void row_end(Row &, int, int, int) const {}
+  __device__ void row_end(Row &r, int b, int t, int s0) const {
+    weak[((size_t)b * ((S + kPairTile) / kPairTile) + s0 / kPairTile) * T + t] = r.weak;
+  }
   // per-column data of a tile in the warp's 4 KB of shared memory: one 16-byte entry
-  // (lmmax, lm[blank], lm[symbol], lm-only normalizer) and the symbol per lattice row
+  // (lmmax, lm[blank], lm[symbol], lm-only normalizer), the symbol and the row's share of the
+  // bound on weak cells per lattice row
   struct Cols {
     float4 q[kPairTile];
     int sym[kPairTile];
+    float bound[kPairTile];
   };
   __device__ void tile_begin(int b, int s0, uint8_t *box, int lane) const {
     Cols *c = reinterpret_cast<Cols *>(box);
@@ -252,6 +255,7 @@ struct NormPairExt {
       const int i = lane + 32 * j, s = s0 + i;
       if (s < S1) {
         const size_t bs = (size_t)b * S1 + s;
+        c->bound[i] = weak_bound(lmsum[bs], 0.f);
         long long y = blank;
         float ls_ = 0.f;
         if (s < S) {
@@ -292,6 +296,7 @@ struct NormPairExt {
     const bool am_on = smoothed && !am_only_off;
     const float lu_blank = am_on ? loguni[blank] : 0.f;
     const float am_y = am_on ? (r.am_blk_t + lu_blank - r.amonly_t) * as : 0.f;
+    float zmin = INFINITY;  // of z less the row's share of the bound
 #pragma unroll
     for (int i = 31; i >= 0; --i, nrow -= T, yrow -= T, xrow -= T1) {
       const int s = s0 + c0 + i;
@@ -299,6 +304,7 @@ struct NormPairExt {
       const float acc = i < 16 ? v0[i & 15] : v1[i & 15];
       const float4 q = c->q[c0 + i];
       const float z = acc * kExpInv2 + 1.17549435e-38f;
+      zmin = fminf(zmin, z - c->bound[c0 + i]);
       const float nv = (EXACT ? logf(z) : __logf(z)) + q.x + r.ammax_t;
       *nrow = nv;
       float vy = r.am_blk_t + q.y - nv;
@@ -320,6 +326,7 @@ struct NormPairExt {
       }
       r.py_next = vy;
     }
+    r.weak |= zmin < weak_bound(0.f, r.am_sum_t);
   }
 };
 
@@ -344,16 +351,16 @@ struct PlaneRow {
   }
 };
 
-// dlm[s][c] = -L[s][c] * sum_t Rw[s][t] A[t][c]  (+ lm-only / unigram terms)
+// dlm[s][c] = -L[s][c] * sum_t Rw[s][t] A[t][c]  (+ lm-only term)
 template <bool ROW_STORE>
 struct LmGradPairExt {
   static constexpr bool kBatched = true, kCustomStore = false, kRowStore = ROW_STORE;
   static constexpr int kGroup = ROW_STORE ? 1 : kPairGroup;
   const __half *lp_hi, *lp_lo;
-  const float *inv_rw, *lmsum, *gl, *dp, *rowdot;
-  int S1, C, Cp;
+  const float *inv_rw, *lmsum, *gl;
+  int S1, Cp;
   struct Row {
-    float sc, inv_sum, g, rd;
+    float sc, inv_sum, g;
     PlaneRow pl;
   };
   __device__ void row_begin(Row &r, int b, int s, int n0) const {
@@ -361,14 +368,13 @@ struct LmGradPairExt {
     r.sc = *inv_rw * (1.f / kExpScale);
     r.inv_sum = gl != nullptr ? 1.f / lmsum[row] : 0.f;
     r.g = gl != nullptr ? gl[row] : 0.f;
-    r.rd = (gl != nullptr && dp != nullptr) ? rowdot[row] : 0.f;
     (void)n0;
   }
   // the planes are padded to whole 64-entry blocks, so a box is always readable
   __device__ void prefetch(Row &r, int b, int s, int n) const {
     if (n < Cp) r.pl.load(lp_hi, lp_lo, ((size_t)b * S1 + s) * Cp + n);
   }
-  __device__ void finish(Row &r, int, int, int c0, float (&v)[16], int half) const {
+  __device__ void finish(Row &r, int, int, int, float (&v)[16], int half) const {
     float L[16];
     r.pl.get(half, L);
 #pragma unroll
@@ -377,7 +383,6 @@ struct LmGradPairExt {
       if (gl != nullptr) {
         const float P = L[i] * r.inv_sum;
         o -= r.g * P;
-        if (dp != nullptr && c0 + i < C) o += P * (dp[c0 + i] - r.rd);
       }
       v[i] = o;
     }
@@ -402,7 +407,8 @@ struct AmGradPairExt {
   __device__ void row_begin(Row &r, int b, int t, int) const {
     const size_t row = (size_t)b * T + t;
     r.sc = *inv_rw * (1.f / kExpScale);
-    r.w = h != nullptr ? h[row] * expf(ammax[row] - amonly[row]) : 0.f;
+    // a weak frame gets the term in float32 later
+    r.w = h != nullptr && !am_only_weak(ammax[row], amonly[row]) ? h[row] * expf(ammax[row] - amonly[row]) : 0.f;
   }
   __device__ void prefetch(Row &r, int b, int t, int n) const {
     if (n < Cp) r.pl.load(ap_hi, ap_lo, ((size_t)b * T + t) * Cp + n);
@@ -422,12 +428,12 @@ struct AmGradPairExt {
   __device__ void tile_begin(int, int, uint8_t *, int) const {}
 };
 
-// Rw [rows][Tp] float -> planes [rows][Tq], columns Tp..Tq-1 zero (they are inside the
+// Rw [rows][Tp] float without the weak cells -> planes [rows][Tq], columns Tp..Tq-1 zero (they are inside the
 // tensor maps only as padding up to T, never beyond it, but the backward's second product
 // reads rows as its reduction index and must not meet stale data)
 __global__ void __launch_bounds__(256)
-sp_split_kernel(const float *__restrict__ x, long long rows, int Tp, int Tq,
-                const float *__restrict__ part, int nparts, __half *__restrict__ hi,
+sp_split_kernel(const float *__restrict__ x, const unsigned *__restrict__ weak, long long rows, int Tp, int Tq,
+                int weak_words, const float *__restrict__ part, int nparts, __half *__restrict__ hi,
                 __half *__restrict__ lo, float *__restrict__ inv_scale) {
   // the maxima of all rows by all threads of every CTA, four entries at a time after that: read
   // by one warp, and split entry by entry with a 64-bit division each, 64 x 101 rows of 500
@@ -451,7 +457,8 @@ sp_split_kernel(const float *__restrict__ x, long long rows, int Tp, int Tq,
     uint2 h = make_uint2(0u, 0u), l = h;
     if (c < Tp) {
       const float4 q = *reinterpret_cast<const float4 *>(x + r * Tp + c);
-      const float v[4] = {q.x, q.y, q.z, q.w};
+      const unsigned w = weak[r * weak_words + c / 32] >> (c % 32);
+      const float v[4] = {w & 1u ? 0.f : q.x, w & 2u ? 0.f : q.y, w & 4u ? 0.f : q.z, w & 8u ? 0.f : q.w};
       fp16_pair4(v, scale, h, l);
     }
     *reinterpret_cast<uint2 *>(hi + 4 * i) = h;
@@ -471,7 +478,7 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
   __half *ap_hi = (__half *)(sv + L.ap_hi), *ap_lo = (__half *)(sv + L.ap_lo);
   float *lm_blk = (float *)(sv + L.lm_blk), *lm_sym = (float *)(sv + L.lm_sym);
   float *lnorm = (float *)(sv + L.lnorm), *am_blk = (float *)(sv + L.am_blk);
-  float *am_sym = (float *)(sv + L.am_sym);
+  float *am_sym = (float *)(sv + L.am_sym), *am_sum = (float *)(sv + L.am_sum);
   const int S1 = S + 1;
   if (stage == 0) {
     const long long rows_lm = (long long)B * S1, rows = rows_lm + (long long)B * T;
@@ -480,7 +487,7 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
   FRNNT_KERNEL(exp_planes_kernel<TIn, VEC, G, K>                                                                    \
                <<<(int)std::min<long long>((((LAST) - (FIRST)) * G + 7) / 8, (long long)sm_count() * 32), 256, 0, st>>>( \
                    (const TIn *)lm, (const TIn *)am, symbols, lp_hi, lp_lo, ap_hi, ap_lo, lmmax, lmsum, ammax,      \
-                   lm_blk, lm_sym, lnorm, am_blk, am_sym, px, B, S, T, C, L.Cp, L.Sp, blank,                        \
+                   lm_blk, lm_sym, lnorm, am_blk, am_sym, am_sum, px, B, S, T, C, L.Cp, L.Sp, blank,                        \
                    rnnt_type == FRNNT_REGULAR, FIRST, LAST))
     // Rows up to 512: lanes keep 16 entries.  Longer rows: lm, whose sum of exponentials counts,
     // stays with one warp per row (the order of that sum is kept); am, by far the most rows, goes
@@ -531,20 +538,23 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
                        (S1 + kPairTile - 1) / kPairTile, B};
   // the policy stores the lattices itself; the engine's output map is unused and is made
   // over the normalizer buffer only because it has to be a valid map
+  const SimpleLattice lattice{
+      norm,   px,     py,    am_sym,  symbols, boundary, lmmax,     ammax,    lm_blk, lm_sym,      lnorm, am_blk,
+      amonly, loguni, lmsum, am_sum,  sv + L.weak, S, T, C, blank,  rnnt_type, smoothed, am_only_off, both,  ls,
+      as,     L.Sp,   delay_penalty};
   auto product = [&](auto exact) {
-    const NormPairExt<decltype(exact)::value> ext{
-        norm,   px,     py,     am_sym,      symbols, boundary, lmmax, ammax,       lm_blk, lm_sym,       lnorm,
-        am_blk, amonly, loguni, S,           T,       C,        blank, rnnt_type,   smoothed, am_only_off, both,
-        ls,     as,     L.Sp,   delay_penalty};
-    return launch_pair_umma<false, false>(mah, mal, mbh, mbl, norm, shape, ext, st);
+    return launch_pair_umma<false, false>(mah, mal, mbh, mbl, norm, shape,
+                                          NormPairExt<decltype(exact)::value>{lattice}, st);
   };
-  return C % 4 == 0 ? product(std::false_type{}) : product(std::true_type{});
+  rc = C % 4 == 0 ? product(std::false_type{}) : product(std::true_type{});
+  if (rc != FRNNT_OK) return rc;
+  return launch_weak_cells(lm, am, input_dtype, lattice, B, st);
 }
 
-int launch_simple_grads_pairs(const float *rw, const float *lmsum, const float *ammax, const float *amonly,
-                              const float *uni, const float *gl, const float *h, const float *dp,
-                              const float *rowdot, float *lm_grad, float *am_grad, const void *pairs_saved,
-                              void *pairs_scratch, int B, int S, int T, int C, int Tp, cudaStream_t st) {
+int launch_simple_grads_pairs(const float *rw, const unsigned *weak, const float *lmsum, const float *ammax,
+                              const float *amonly, const float *uni, const float *gl, const float *h,
+                              float *lm_grad, float *am_grad, const void *pairs_saved, void *pairs_scratch, int B, int S, int T, int C, int Tp,
+                              cudaStream_t st) {
   const SimplePairsLayout L(B, S, T, C);
   const uint8_t *sv = (const uint8_t *)pairs_saved;
   uint8_t *sc = (uint8_t *)pairs_scratch;
@@ -570,7 +580,7 @@ int launch_simple_grads_pairs(const float *rw, const float *lmsum, const float *
   const int nparts = (int)rows;
   const long long nq = rows * (Tq / 4);
   const int grid = (int)std::min<long long>((nq + 255) / 256, (long long)sm_count() * 16);
-  FRNNT_KERNEL(sp_split_kernel<<<grid, 256, 0, st>>>(rw, rows, Tp, Tq, parts, nparts, rw_hi, rw_lo, inv_rw));
+  FRNNT_KERNEL(sp_split_kernel<<<grid, 256, 0, st>>>(rw, weak, rows, Tp, Tq, weak_words(T), parts, nparts, rw_hi, rw_lo, inv_rw));
   FRNNT_CUDA(cudaGetLastError());
 
   const int ctiles = (C + kPairTile - 1) / kPairTile;
@@ -578,7 +588,7 @@ int launch_simple_grads_pairs(const float *rw, const float *lmsum, const float *
   const LinShape am_shape{T, C, S1, ((S1 + kPairBK - 1) / kPairBK) * kPairBK, (T + kPairTile - 1) / kPairTile, ctiles, B};
   auto products = [&](auto row_store) {
     constexpr bool kRow = decltype(row_store)::value;
-    const LmGradPairExt<kRow> lm_ext{lp_hi, lp_lo, inv_rw, lmsum, gl, dp, rowdot, S1, C, Cp};
+    const LmGradPairExt<kRow> lm_ext{lp_hi, lp_lo, inv_rw, lmsum, gl, S1, Cp};
     const int r = launch_pair_umma<false, true>(a1h, a1l, b1h, b1l, lm_grad, lm_shape, lm_ext, st);
     if (r != FRNNT_OK) return r;
     const AmGradPairExt<kRow> am_ext{ap_hi, ap_lo, inv_rw, ammax, h, uni, amonly, T, C, Cp};
