@@ -812,7 +812,7 @@ __global__ void grad_weight_kernel(EffGrads<real> eg, const real *__restrict__ n
 
 // The two kernels above and below in one pass, for the tensor-core path: one CTA per lattice
 // row (b, s) writes the row of Rw, the row sums of gx (all T1 columns) and gy, and the
-// row's largest |Rw| (which sets the scale of the fp16 planes Rw is split into).  Weak cells
+// row's largest finite |Rw| (which sets the scale of the fp16 planes Rw is split into).  Weak cells
 // (simple_pairs.cuh) do not go into the planes: their bits go to `weak`, weak_row says whether
 // the row has any.
 template <typename real>
@@ -847,7 +847,7 @@ grad_weight_rows_kernel(EffGrads<real> eg, const real *__restrict__ norm, const 
           is_weak = w != 0 && (float)inv * weak_bound(lms, am_sum[(size_t)b * eg.T + t]) > 1.f;
         }
         rw[(size_t)row * Tp + t] = v;
-        if (!is_weak) mx = max(mx, v < 0 ? -v : v);
+        if (!is_weak && v - v == 0) mx = max(mx, v < 0 ? -v : v);
       }
     }
     const unsigned bits = __ballot_sync(0xffffffffu, is_weak);

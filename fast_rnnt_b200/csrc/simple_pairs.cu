@@ -59,7 +59,7 @@ SimplePairsLayout::SimplePairsLayout(int B, int S, int T, int C) {
   rw_hi = take((size_t)B * S1 * Tq * 2);
   rw_lo = take((size_t)B * S1 * Tq * 2);
   parts = take(std::max<size_t>(kSpParts, (size_t)B * S1) * 4);
-  inv_scale = take(64);
+  inv_scale = take((size_t)B * 4);
   scratch_bytes = o;
 }
 
@@ -365,7 +365,7 @@ struct LmGradPairExt {
   };
   __device__ void row_begin(Row &r, int b, int s, int n0) const {
     const size_t row = (size_t)b * S1 + s;
-    r.sc = *inv_rw * (1.f / kExpScale);
+    r.sc = inv_rw[b] * (1.f / kExpScale);
     r.inv_sum = gl != nullptr ? 1.f / lmsum[row] : 0.f;
     r.g = gl != nullptr ? gl[row] : 0.f;
     (void)n0;
@@ -406,7 +406,7 @@ struct AmGradPairExt {
   };
   __device__ void row_begin(Row &r, int b, int t, int) const {
     const size_t row = (size_t)b * T + t;
-    r.sc = *inv_rw * (1.f / kExpScale);
+    r.sc = inv_rw[b] * (1.f / kExpScale);
     // a weak frame gets the term in float32 later
     r.w = h != nullptr && !am_only_weak(ammax[row], amonly[row]) ? h[row] * expf(ammax[row] - amonly[row]) : 0.f;
   }
@@ -428,41 +428,42 @@ struct AmGradPairExt {
   __device__ void tile_begin(int, int, uint8_t *, int) const {}
 };
 
-// Rw [rows][Tp] float without the weak cells -> planes [rows][Tq], columns Tp..Tq-1 zero (they are inside the
-// tensor maps only as padding up to T, never beyond it, but the backward's second product
-// reads rows as its reduction index and must not meet stale data)
+// Rw [B][S1][Tp] float without the weak cells -> planes [B][S1][Tq], columns Tp..Tq-1 zero (they are
+// inside the tensor maps only as padding up to T, never beyond it, but the backward's second product
+// reads rows as its reduction index and must not meet stale data).  One scale per utterance
+// (blockIdx.y), so that its planes do not depend on the weights of the others.
 __global__ void __launch_bounds__(256)
-sp_split_kernel(const float *__restrict__ x, const unsigned *__restrict__ weak, long long rows, int Tp, int Tq,
-                int weak_words, const float *__restrict__ part, int nparts, __half *__restrict__ hi,
+sp_split_kernel(const float *__restrict__ x, const unsigned *__restrict__ weak, int S1, int Tp, int Tq,
+                int weak_words, const float *__restrict__ part, __half *__restrict__ hi,
                 __half *__restrict__ lo, float *__restrict__ inv_scale) {
-  // the maxima of all rows by all threads of every CTA, four entries at a time after that: read
-  // by one warp, and split entry by entry with a 64-bit division each, 64 x 101 rows of 500
-  // took 19.5 us; 10.8 us this way
+  // the maxima of the utterance's rows by all threads of each of its CTAs, four entries at a time
+  // after that: 64 x 101 rows of 500 in 9.0 us (11.2 with one scale, i.e. every CTA reading all maxima)
   __shared__ float slot[8];
+  const size_t row0 = (size_t)blockIdx.y * S1;
   float m = 0.f;
 #pragma unroll 4
-  for (int i = threadIdx.x; i < nparts; i += 256) m = fmaxf(m, part[i]);
+  for (int i = threadIdx.x; i < S1; i += 256) m = fmaxf(m, part[row0 + i]);
   m = warp_max(m);
   if ((threadIdx.x & 31) == 0) slot[threadIdx.x >> 5] = m;
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < 8; ++w) m = fmaxf(m, slot[w]);
   const float scale = fp16_pair_scale(m);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *inv_scale = 1.f / scale;
+  if (blockIdx.x == 0 && threadIdx.x == 0) inv_scale[blockIdx.y] = 1.f / scale;
   const int nvec = Tq / 4;  // Tp is a multiple of 4, too
-  const long long n = rows * nvec;
+  const long long n = (long long)S1 * nvec;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-    const long long r = div_rows(i, nvec);
-    const int c = 4 * (int)(i - r * nvec);
+    const size_t r = row0 + div_rows(i, nvec);
+    const int q = mod_rows(i, nvec), c = 4 * q;
     uint2 h = make_uint2(0u, 0u), l = h;
     if (c < Tp) {
-      const float4 q = *reinterpret_cast<const float4 *>(x + r * Tp + c);
+      const float4 q4 = *reinterpret_cast<const float4 *>(x + r * Tp + c);
       const unsigned w = weak[r * weak_words + c / 32] >> (c % 32);
-      const float v[4] = {w & 1u ? 0.f : q.x, w & 2u ? 0.f : q.y, w & 4u ? 0.f : q.z, w & 8u ? 0.f : q.w};
+      const float v[4] = {w & 1u ? 0.f : q4.x, w & 2u ? 0.f : q4.y, w & 4u ? 0.f : q4.z, w & 8u ? 0.f : q4.w};
       fp16_pair4(v, scale, h, l);
     }
-    *reinterpret_cast<uint2 *>(hi + 4 * i) = h;
-    *reinterpret_cast<uint2 *>(lo + 4 * i) = l;
+    reinterpret_cast<uint2 *>(hi)[r * nvec + q] = h;
+    reinterpret_cast<uint2 *>(lo)[r * nvec + q] = l;
   }
 }
 
@@ -563,7 +564,6 @@ int launch_simple_grads_pairs(const float *rw, const unsigned *weak, const float
   __half *rw_hi = (__half *)(sc + L.rw_hi), *rw_lo = (__half *)(sc + L.rw_lo);
   float *parts = (float *)(sc + L.parts), *inv_rw = (float *)(sc + L.inv_scale);
   const int S1 = S + 1, Cp = L.Cp, Tq = L.Tq;
-  const long long rows = (long long)B * S1;
 
   CUtensorMap a1h, a1l, b1h, b1l, a2h, a2l, b2h, b2l;
   int rc = make_pair_map(&a1h, rw_hi, S1, T, Tq, false, B, (long long)S1 * Tq);      // Rw [s][t], K = t
@@ -577,10 +577,9 @@ int launch_simple_grads_pairs(const float *rw, const unsigned *weak, const float
   if (rc != FRNNT_OK) return rc;
 
   // the caller left max |rw| per row in `parts`
-  const int nparts = (int)rows;
-  const long long nq = rows * (Tq / 4);
-  const int grid = (int)std::min<long long>((nq + 255) / 256, (long long)sm_count() * 16);
-  FRNNT_KERNEL(sp_split_kernel<<<grid, 256, 0, st>>>(rw, weak, rows, Tp, Tq, weak_words(T), parts, nparts, rw_hi, rw_lo, inv_rw));
+  const long long per_utt = ((long long)S1 * (Tq / 4) + 255) / 256;
+  const dim3 grid((unsigned)std::min(per_utt, std::max<long long>(1, (long long)sm_count() * 16 / B)), (unsigned)B);
+  FRNNT_KERNEL(sp_split_kernel<<<grid, 256, 0, st>>>(rw, weak, S1, Tp, Tq, weak_words(T), parts, rw_hi, rw_lo, inv_rw));
   FRNNT_CUDA(cudaGetLastError());
 
   const int ctiles = (C + kPairTile - 1) / kPairTile;

@@ -110,3 +110,44 @@ def test_beyond_the_range_of_float32(monkeypatch, C):
     ref = lattices(lm, am, symbols, "regular", (0.0, 0.0), C)
     for a, b in zip(got, ref):
         torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("C", [51, 52])
+@pytest.mark.parametrize("weight", [1e10, float("inf"), float("nan")])
+@pytest.mark.parametrize("peaked", [False, True])
+def test_gradients_do_not_depend_on_the_other_utterances(C, weight, peaked):
+    import fast_rnnt_b200 as fr
+    torch.manual_seed(C)
+    lm, am = torch.randn(3, 21, C).cuda(), torch.randn(3, 40, C).cuda()
+    symbols = torch.randint(1, C, (3, 20)).cuda()
+    if peaked:
+        lm[1], am[1] = 0, 0
+        lm[1, :, 3], am[1, :, 5] = 20, 20
+    lm.requires_grad_(True)
+    am.requires_grad_(True)
+    px, py = fr.get_rnnt_logprobs(lm, am, symbols, 0)
+    gx, gy = torch.rand_like(px), torch.rand_like(py)
+    alone = torch.autograd.grad([px, py], [lm, am], [gx, gy], retain_graph=True)
+    gx[1] *= weight
+    gy[1] *= weight
+    beside = torch.autograd.grad([px, py], [lm, am], [gx, gy])
+    for a, b in zip(alone, beside):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[2], b[2])
+
+
+@pytest.mark.parametrize("C", [51, 52])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_a_cell_without_a_finite_gradient_spoils_its_row_and_frame_only(C, value):
+    import fast_rnnt_b200 as fr
+    torch.manual_seed(C)
+    lm = torch.randn(1, 21, C).cuda().requires_grad_(True)
+    am = torch.randn(1, 40, C).cuda().requires_grad_(True)
+    px, py = fr.get_rnnt_logprobs(lm, am, torch.randint(1, C, (1, 20)).cuda(), 0)
+    gx, gy = torch.rand_like(px) * 1e-3, torch.rand_like(py) * 1e-3
+    alone = torch.autograd.grad([px, py], [lm, am], [gx, gy], retain_graph=True)
+    gx[0, 4, 7] = value
+    beside = torch.autograd.grad([px, py], [lm, am], [gx, gy])
+    for a, b, i in zip(alone, beside, (4, 7)):
+        others = [k for k in range(a.shape[1]) if k != i]
+        torch.testing.assert_close(a[0, others], b[0, others], rtol=1e-6, atol=1e-9)
+        assert not torch.isfinite(b[0, i]).all()
