@@ -1275,7 +1275,8 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
     rc = launch_simple_grads_pairs((const float *)rw, weak, (const float *)lmsum, (const float *)ammax,
                                    (const float *)amonly, (const float *)uni, (const float *)gl_p,
                                    (const float *)h_p, (float *)lm_grad, (float *)am_grad, svb + sv.total,
-                                   scb + sc.total, B, S, T, C, Tp, st);
+                                   scb + sc.total, B, S, T, C, Tp,
+                                   simple_pairs_exact(lm_, am_, C, input_dtype), st);
     if (rc != FRNNT_OK) return rc;
     if (dp_p != nullptr)
       FRNNT_KERNEL(lm_unigram_grad_kernel<<<(unsigned)lm_rows, 256, 0, st>>>(

@@ -83,6 +83,18 @@ static bool rows_by_four(const void *a, const void *b, int C) {
   return C % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)b % 16 == 0;
 }
 
+// Which calls get the more accurate form of the products (EXACT: a fresh accumulator per 64 values of
+// the reduction instead of 128, the small products first): those whose rows of 4-byte values
+// are not all 16-byte aligned.  The FMA pipe used to serve them, and its float32 sums are more
+// accurate than 128 truncating tensor-core additions.  Relative errors of px and of the am
+// gradient in 1e-8, 160 x 41 cells of unit normals, C = 64 / 128 / 500: in groups of 128 8.1,
+// 14.2, 11.9 and 9.0, 16.8, 10.2; in groups of 64 6.0, 5.5, 4.9 and 7.9, 7.0, 6.1; on the FMA pipe
+// 4.9, 4.9, 6.0 and 7.4, 6.7, 6.1.  16-bit rows get what their float32 copies get, which are
+// aligned.
+bool simple_pairs_exact(const void *lm, const void *am, int C, int input_dtype) {
+  return is_half_input(input_dtype) ? C % 4 != 0 : !rows_by_four(lm, am, C);
+}
+
 // ---- forward, pass 1: row maxima, exp planes, per-row scalars -----------------------------------
 // entries 4 v .. 4 v + 3 of a row of C; VEC: as one load, else singly, -inf beyond the row (exp: 0)
 template <bool VEC, typename TIn>
@@ -209,9 +221,8 @@ exp_planes_kernel(const TIn *__restrict__ lm, const TIn *__restrict__ am,
 
 // ---- forward, pass 2: the normalizer product and the lattices ----------------------------------
 // tile rows = frames t, tile columns = lattice rows s
-// EXACT: a fresh accumulator per 64 values of the reduction and logf instead of __logf.  For the
-// vocabularies that the FMA pipe used to serve, whose float32 sums were more accurate than 128
-// truncating tensor-core additions (C = 50 .. 500: relative error of px 1.0e-7 against 5.5e-8)
+// EXACT (simple_pairs_exact): a fresh accumulator per 64 values of the reduction and logf instead of
+// __logf
 template <bool EXACT>
 struct NormPairExt : SimpleLattice {
   static constexpr bool kBatched = true, kCustomStore = true;
@@ -352,10 +363,10 @@ struct PlaneRow {
 };
 
 // dlm[s][c] = -L[s][c] * sum_t Rw[s][t] A[t][c]  (+ lm-only term)
-template <bool ROW_STORE>
+template <bool ROW_STORE, bool EXACT>
 struct LmGradPairExt {
   static constexpr bool kBatched = true, kCustomStore = false, kRowStore = ROW_STORE;
-  static constexpr int kGroup = ROW_STORE ? 1 : kPairGroup;
+  static constexpr int kGroup = EXACT ? 1 : kPairGroup;
   const __half *lp_hi, *lp_lo;
   const float *inv_rw, *lmsum, *gl;
   int S1, Cp;
@@ -393,10 +404,10 @@ struct LmGradPairExt {
 };
 
 // dam[t][c] = -A[t][c] * sum_s Rw[s][t] L[s][c]  (+ am-only term)
-template <bool ROW_STORE>
+template <bool ROW_STORE, bool EXACT>
 struct AmGradPairExt {
   static constexpr bool kBatched = true, kCustomStore = false, kRowStore = ROW_STORE;
-  static constexpr int kGroup = ROW_STORE ? 1 : kPairGroup;
+  static constexpr int kGroup = EXACT ? 1 : kPairGroup;
   const __half *ap_hi, *ap_lo;
   const float *inv_rw, *ammax, *h, *uni, *amonly;
   int T, C, Cp;
@@ -547,7 +558,7 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
     return launch_pair_umma<false, false>(mah, mal, mbh, mbl, norm, shape,
                                           NormPairExt<decltype(exact)::value>{lattice}, st);
   };
-  rc = C % 4 == 0 ? product(std::false_type{}) : product(std::true_type{});
+  rc = simple_pairs_exact(lm, am, C, input_dtype) ? product(std::true_type{}) : product(std::false_type{});
   if (rc != FRNNT_OK) return rc;
   return launch_weak_cells(lm, am, input_dtype, lattice, B, st);
 }
@@ -555,7 +566,7 @@ int launch_simple_forward_pairs(const void *lm, const void *am, const int64_t *s
 int launch_simple_grads_pairs(const float *rw, const unsigned *weak, const float *lmsum, const float *ammax,
                               const float *amonly, const float *uni, const float *gl, const float *h,
                               float *lm_grad, float *am_grad, const void *pairs_saved, void *pairs_scratch, int B, int S, int T, int C, int Tp,
-                              cudaStream_t st) {
+                              bool exact, cudaStream_t st) {
   const SimplePairsLayout L(B, S, T, C);
   const uint8_t *sv = (const uint8_t *)pairs_saved;
   uint8_t *sc = (uint8_t *)pairs_scratch;
@@ -585,15 +596,17 @@ int launch_simple_grads_pairs(const float *rw, const unsigned *weak, const float
   const int ctiles = (C + kPairTile - 1) / kPairTile;
   const LinShape lm_shape{S1, C, T, ((T + kPairBK - 1) / kPairBK) * kPairBK, (S1 + kPairTile - 1) / kPairTile, ctiles, B};
   const LinShape am_shape{T, C, S1, ((S1 + kPairBK - 1) / kPairBK) * kPairBK, (T + kPairTile - 1) / kPairTile, ctiles, B};
-  auto products = [&](auto row_store) {
-    constexpr bool kRow = decltype(row_store)::value;
-    const LmGradPairExt<kRow> lm_ext{lp_hi, lp_lo, inv_rw, lmsum, gl, S1, Cp};
+  auto products = [&](auto row_store, auto more_exact) {
+    constexpr bool kRow = decltype(row_store)::value, kExact = decltype(more_exact)::value;
+    const LmGradPairExt<kRow, kExact> lm_ext{lp_hi, lp_lo, inv_rw, lmsum, gl, S1, Cp};
     const int r = launch_pair_umma<false, true>(a1h, a1l, b1h, b1l, lm_grad, lm_shape, lm_ext, st);
     if (r != FRNNT_OK) return r;
-    const AmGradPairExt<kRow> am_ext{ap_hi, ap_lo, inv_rw, ammax, h, uni, amonly, T, C, Cp};
+    const AmGradPairExt<kRow, kExact> am_ext{ap_hi, ap_lo, inv_rw, ammax, h, uni, amonly, T, C, Cp};
     return launch_pair_umma<true, true>(a2h, a2l, b2h, b2l, am_grad, am_shape, am_ext, st);
   };
-  return rows_by_four(lm_grad, am_grad, C) ? products(std::false_type{}) : products(std::true_type{});
+  // TMA stores where the gradients' rows allow them, whatever the rows of lm and am
+  if (!rows_by_four(lm_grad, am_grad, C)) return products(std::true_type{}, std::true_type{});
+  return exact ? products(std::false_type{}, std::true_type{}) : products(std::false_type{}, std::false_type{});
 }
 
 }  // namespace frnnt

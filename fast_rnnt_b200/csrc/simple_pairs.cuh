@@ -38,6 +38,9 @@ size_t simple_pairs_rowmax_offset(int B, int S, int T, int C);
 
 bool simple_pairs_supported(const void *lm, const void *am, int S1, int T, int C, int rnnt_type);
 
+// whether a call gets the more accurate form of the products
+bool simple_pairs_exact(const void *lm, const void *am, int C, int input_dtype);
+
 // stage 0: row maxima / sums, exp planes, per-row scalars, the -inf column of px;
 // stage 1: normalizer product + lattices (needs amonly / loguni when the am-only branch is on;
 // a positive delay_penalty is added to px as the reference's loss functions do)
@@ -76,6 +79,6 @@ __host__ __device__ inline int weak_words(int T) { return (T + 31) / 32; }
 int launch_simple_grads_pairs(const float *rw, const unsigned *weak, const float *lmsum, const float *ammax,
                               const float *amonly, const float *uni, const float *gl, const float *h,
                               float *lm_grad, float *am_grad, const void *pairs_saved, void *pairs_scratch, int B, int S, int T, int C, int Tp,
-                              cudaStream_t st);
+                              bool exact, cudaStream_t st);
 
 }  // namespace frnnt
