@@ -1082,9 +1082,15 @@ int launch_simple_grads_umma(const float *lm, const float *am, const float *lmma
                              const float *dp, const float *rowdot, float *lm_grad, float *am_grad,
                              int B, int S1, int T, int C, int Tp, cudaStream_t st);
 
+// buffers of the caller's that only the FMA pipe, which moves single values, can work in
+static bool off_16_bytes(const void *saved, const void *scratch) {
+  return (uintptr_t)saved % 16 != 0 || (uintptr_t)scratch % 16 != 0;
+}
+
 template <typename real>
-static bool use_tensor_cores(const void *lm, const void *am, int S1, int T, int C) {
-  if (sizeof(real) != 4) return false;
+static bool use_tensor_cores(const void *lm, const void *am, const void *saved, const void *scratch, int S1, int T,
+                             int C) {
+  if (sizeof(real) != 4 || off_16_bytes(saved, scratch)) return false;
   const char *mode = getenv("FRNNT_CONTRACTION");
   if (mode != nullptr && strcmp(mode, "simt") == 0) return false;
   return norm_umma_supported(lm, am, S1, T, C);
@@ -1092,8 +1098,9 @@ static bool use_tensor_cores(const void *lm, const void *am, int S1, int T, int 
 
 // the fp16-pair engine (FRNNT_CONTRACTION=tf32 keeps the 3xTF32 kernels, =simt the FMA pipe)
 template <typename real>
-static bool use_pairs(const void *lm, const void *am, int S1, int T, int C, int rnnt_type) {
-  if (sizeof(real) != 4) return false;
+static bool use_pairs(const void *lm, const void *am, const void *saved, const void *scratch, int S1, int T, int C,
+                      int rnnt_type) {
+  if (sizeof(real) != 4 || off_16_bytes(saved, scratch)) return false;
   const char *mode = getenv("FRNNT_CONTRACTION");
   if (mode != nullptr && (strcmp(mode, "simt") == 0 || strcmp(mode, "tf32") == 0)) return false;
   return simple_pairs_supported(lm, am, S1, T, C, rnnt_type);
@@ -1148,7 +1155,7 @@ static int simple_forward_impl(const void *lm_, const void *am_, const int64_t *
   real *loguni = (real *)(svb + sv.loguni), *partial = (real *)(scb + sc.partial);
   const long long lm_rows = (long long)B * S1, am_rows = (long long)B * T;
 
-  const bool pairs = use_pairs<real>(lm, am, S1, T, C, rnnt_type);
+  const bool pairs = use_pairs<real>(lm, am, saved, nullptr, S1, T, C, rnnt_type);
   FRNNT_REQUIRE(!is_half_input(input_dtype) || (pairs && (!cfg.smoothed || cfg.am_only_off)), FRNNT_EUNSUPPORTED,
                 "16-bit inputs are read by the tensor-core path without the am-only branch only "
                 "(frnnt_simple_reads_16bit_inputs)");
@@ -1184,7 +1191,7 @@ static int simple_forward_impl(const void *lm_, const void *am_, const int64_t *
                                        (float *)lmmax, (float *)lmsum, (float *)ammax, (const float *)amonly,
                                        (const float *)loguni, pairs_saved, B, S, T, C, 1, st, cfg.delay_penalty,
                                        input_dtype);
-  if (use_tensor_cores<real>(lm, am, S1, T, C)) {
+  if (use_tensor_cores<real>(lm, am, saved, nullptr, S1, T, C)) {
     rc = launch_norm_umma((const float *)lm, (const float *)am, (const float *)lmmax,
                           (const float *)ammax, (float *)norm, B, S1, T, C, st);
   } else {
@@ -1226,7 +1233,7 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
   EffGrads<real> eg{(const real *)px_grad, (const real *)py_grad, boundary, S, T, T1, rnnt_type};
 
   const int Tp = rw_pitch(T);
-  const bool pairs = use_pairs<real>(lm, am, S1, T, C, rnnt_type) && T > 0;
+  const bool pairs = use_pairs<real>(lm, am, saved, scratch, S1, T, C, rnnt_type) && T > 0;
   dim3 g3((unsigned)((Tp + 127) / 128), (unsigned)S1, (unsigned)B);
   const float *am_sum = (const float *)(svb + sv.total + simple_pairs_amsum_offset(B, S, T, C));
   unsigned *weak = (unsigned *)(scb + sc.weak);
@@ -1297,7 +1304,7 @@ static int simple_backward_impl(const void *lm_, const void *am_, const int64_t 
       FRNNT_KERNEL(weak_grads_kernel<<<ctas, kWeakThreads, 0, st>>>(g, lm_split, am_split));
     });
     FRNNT_CUDA(cudaGetLastError());
-  } else if (use_tensor_cores<real>(lm, am, S1, T, C)) {
+  } else if (use_tensor_cores<real>(lm, am, saved, scratch, S1, T, C)) {
     rc = launch_simple_grads_umma((const float *)lm, (const float *)am, (const float *)lmmax,
                                   (const float *)lmsum, (const float *)ammax, (const float *)amonly,
                                   (const float *)uni, (const float *)rw, (const float *)gl_p,
@@ -1347,7 +1354,7 @@ extern "C" int frnnt_simple_reads_16bit_inputs(int S, int T, int C, int rnnt_typ
   if (S < 0 || T < 1 || C < 1) return 0;
   if (smoothed && am_only_scale != 0.0) return 0;
   // 256-byte aligned rows stand in for the caller's tensors (torch's allocations are)
-  return use_pairs<float>((const void *)256, (const void *)256, S + 1, T, C, rnnt_type) ? 1 : 0;
+  return use_pairs<float>((const void *)256, (const void *)256, nullptr, nullptr, S + 1, T, C, rnnt_type) ? 1 : 0;
 }
 
 extern "C" int frnnt_simple_logprobs_forward(int dtype, const void *lm, const void *am,
@@ -1392,7 +1399,7 @@ extern "C" int frnnt_simple_logprobs_backward(int dtype, const void *lm, const v
   const int am_only_active = smoothed && am_only_scale != 0.0;
   cudaStream_t st = (cudaStream_t)stream;
   if (is_half_input(dtype)) {
-    FRNNT_REQUIRE(use_pairs<float>(lm, am, S + 1, T, C, rnnt_type) && T > 0 && !am_only_active,
+    FRNNT_REQUIRE(use_pairs<float>(lm, am, saved, scratch, S + 1, T, C, rnnt_type) && T > 0 && !am_only_active,
                   FRNNT_EUNSUPPORTED, "16-bit inputs: see frnnt_simple_reads_16bit_inputs");
   }
   if (dtype != FRNNT_F64)

@@ -92,3 +92,37 @@ def test_unaligned_16_bit_rows_equal_their_float32_copies(dtype):
     ref = lattices(lm.float(), am.float(), symbols, "regular", (0.25, 0.0), C)
     for a, b in zip(got, ref):
         assert torch.equal(a, b.to(a.dtype))
+
+
+@pytest.mark.parametrize("C", [37, 40])
+@pytest.mark.parametrize("offsets", [(4, 0), (0, 4), (4, 4), (16, 16)])
+def test_buffers_off_a_16_byte_boundary(C, offsets):
+    """The caller's saved area and backward scratch through the C ABI: planes and their tensor maps
+    need 16 bytes, other buffers are served in single values."""
+    from fast_rnnt_b200 import _lib
+    from fast_rnnt_b200._lib import _c_f64, _c_int, _c_vp, ptr
+    lib, B, S, T = _lib.lib(), 2, 9, 21
+    torch.manual_seed(C)
+    lm, am = torch.randn(B, S + 1, C).cuda(), torch.randn(B, T, C).cuda()
+    symbols = torch.randint(1, C, (B, S)).cuda()
+    gx, gy = torch.rand(B, S, T + 1).cuda(), torch.rand(B, S + 1, T).cuda()
+    saved_bytes = lib.frnnt_simple_saved_bytes(0, B, S, T, C)
+    scratch_bytes = lib.frnnt_simple_scratch_bytes(0, B, S, T, C)
+
+    def run(off_saved, off_scratch):
+        saved = torch.zeros(saved_bytes + 64, dtype=torch.uint8, device="cuda")
+        scratch = torch.zeros(scratch_bytes + 64, dtype=torch.uint8, device="cuda")
+        sv, sc = _c_vp(saved.data_ptr() + off_saved), _c_vp(scratch.data_ptr() + off_scratch)
+        px, py = torch.empty_like(gx), torch.empty_like(gy)
+        gl, ga = torch.empty_like(lm), torch.empty_like(am)
+        st = _lib.stream_ptr(lm.device)
+        _lib.call("frnnt_simple_logprobs_forward", _c_int(0), ptr(lm), ptr(am), ptr(symbols), None, 0, 0, 0,
+                  _c_f64(0.0), _c_f64(0.0), _c_f64(0.0), ptr(px), ptr(py), sv, sc, B, S, T, C, st)
+        _lib.call("frnnt_simple_logprobs_backward", _c_int(0), ptr(lm), ptr(am), ptr(symbols), None, 0, 0, 0,
+                  _c_f64(0.0), _c_f64(0.0), ptr(gx), ptr(gy), sv, sc, ptr(gl), ptr(ga), B, S, T, C, st)
+        torch.cuda.synchronize()
+        assert not saved[saved_bytes + off_saved:].any() and not scratch[scratch_bytes + off_scratch:].any()
+        return px, py, gl, ga
+
+    for a, b in zip(run(*offsets), run(0, 0)):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
