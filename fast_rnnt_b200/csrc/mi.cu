@@ -855,3 +855,21 @@ extern "C" int frnnt_mi_fwd_bwd_noalloc(int dtype, const void *px, const void *p
   return frnnt_mi_backward_from_lattice(dtype, px, scratch, boundary, ans_grad, px_grad, py_grad,
                                         nullptr, B, S, T, modified, stream);
 }
+
+extern "C" int frnnt_mi_sweeps_limited(const float *px, const float *py, const int64_t *boundary,
+                                       const float *ans_grad, float *p, float *ans, float *px_grad,
+                                       float *py_grad, float *origin_grad, void *lattice, int B, int S, int T,
+                                       int modified, int forward_tries, int backward_tries, void *stream) {
+  int ncw = 0;
+  int rc = mi_check_sizes(FRNNT_F32, B, S, T, modified, &ncw);
+  if (rc != FRNNT_OK) return rc;
+  if (B == 0) return FRNNT_OK;
+  FRNNT_REQUIRE(px && py && ans_grad && ans && px_grad && py_grad && lattice && (uintptr_t)lattice % 16 == 0,
+                FRNNT_EINVAL, "NULL argument or lattice off a 16-byte boundary");
+  cudaStream_t st = (cudaStream_t)stream;
+  rc = launch_mi_forward_f32(px, py, boundary, p, ans, (float *)lattice, B, S, T, modified, st,
+                             forward_tries < 0 ? kMiTries : forward_tries);
+  if (rc != FRNNT_OK) return rc;
+  return launch_mi_backward_f32((float *)lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, modified,
+                                st, backward_tries < 0 ? kMiTries : backward_tries);
+}

@@ -66,11 +66,13 @@ __device__ __forceinline__ double weight_of(double value) { return exp(value); }
 
 // float sweeps (mi_f32.cu).  `lattice` must be 16-byte aligned; the forward takes NULL when
 // the whole lattice fits one launch (S + 1 <= kMiF32Rows) and no backward sweep follows.
-constexpr int kMiF32Rows = 512;
+// `tries` bounds every wait between the CTAs of a cluster.
+constexpr int kMiF32Rows = 512, kMiTries = 1 << 22;
 int launch_mi_forward_f32(const float *px, const float *py, const int64_t *boundary, float *p, float *ans,
-                          float *lattice, int B, int S, int T, int modified, cudaStream_t st);
+                          float *lattice, int B, int S, int T, int modified, cudaStream_t st,
+                          int tries = kMiTries);
 int launch_mi_backward_f32(float *lattice, const int64_t *boundary, const float *ans_grad, float *px_grad,
                            float *py_grad, float *origin_grad, int B, int S, int T, int modified,
-                           cudaStream_t st);
+                           cudaStream_t st, int tries = kMiTries);
 
 }  // namespace frnnt

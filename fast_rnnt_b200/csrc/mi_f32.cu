@@ -104,10 +104,11 @@ __device__ __forceinline__ void peer_send(unsigned address, float v, unsigned ba
 
 // Hand-over of the edge row between neighbouring CTAs, chunks numbered in the order of the sweep.
 // Each side has one mbarrier per slot of the edge ring (chunk mod 8): `full` in the consumer's
-// shared memory, `taken` in the producer's.  Every wait is bounded; one that runs out makes
-// all later ones give up at once (and the caller's results NaN).
+// shared memory, `taken` in the producer's.  Every wait is bounded.  One that runs out makes all
+// later ones of its warp give up at once; the CTA goes on with NaN for the edge row, which the
+// recursion carries to every cell behind it, to the CTAs and row blocks that follow, and so to
+// the score, the remaining gradients and the origin's.
 constexpr int kSlots = kEdgeRing / kStep;
-constexpr int kSpinLimit = 1 << 22;
 
 __device__ __forceinline__ void slot_init(uint64_t *bars) {
   for (int i = 0; i < 2 * kSlots; ++i)
@@ -125,10 +126,11 @@ __device__ __forceinline__ void slot_expect(uint64_t *bars, int chunk, int steps
                "r"(4 * steps)
                : "memory");
 }
-__device__ __forceinline__ bool slot_wait(const uint64_t *bars, int chunk, bool failed) {
+// true: nothing came within `tries` looks (or the warp has given up before)
+__device__ __forceinline__ bool slot_wait(const uint64_t *bars, int chunk, bool failed, int tries) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(bars + chunk % kSlots);
   const unsigned parity = (chunk / kSlots) & 1;
-  for (int spin = 0; !failed; ++spin) {
+  for (int spin = 0; !failed && spin < tries; ++spin) {
     unsigned done;
     asm volatile("{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n"
                  "selp.u32 %0, 1, 0, q;\n}"
@@ -136,11 +138,17 @@ __device__ __forceinline__ bool slot_wait(const uint64_t *bars, int chunk, bool 
                  : "r"(a), "r"(parity)
                  : "memory");
     if (done) return false;
-    failed = spin >= kSpinLimit;
   }
   return true;
 }
 __device__ __forceinline__ void cluster_sync() { cooperative_groups::this_cluster().sync(); }
+// The end of a CTA.  The neighbours may still be writing here until all have arrived; a warp that gave
+// up waiting has not seen its last values arrive, so it stays for 64 us, some fifty times as
+// long as they are under way at most.
+__device__ __forceinline__ void leave_cluster(bool failed) {
+  cluster_sync();
+  for (int i = 0; failed && i < 64; ++i) __nanosleep(1000);
+}
 
 template <int R>
 struct MiShape {
@@ -162,7 +170,7 @@ template <int R, bool CLUSTER, bool MODIFIED, bool WRITE_P, bool BLOCKED>
 __global__ void __launch_bounds__(kThreads)
 mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py,
                       const int64_t *__restrict__ boundary, float *__restrict__ p, float *__restrict__ ans,
-                      float *__restrict__ lattice, int B, int S, int T, int row0_arg) {
+                      float *__restrict__ lattice, int B, int S, int T, int row0_arg, int tries) {
   using M = MiShape<R>;
   constexpr int ROWS = M::kRows, PITCH = M::kRing, G = M::kGroup;
   constexpr int off = MODIFIED ? -1 : 0;
@@ -293,10 +301,11 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
   const unsigned next = has_next ? peer_address(above, rank + 1) : 0u;
   const unsigned next_full = has_next ? peer_address(bars, rank + 1) : 0u;
   const unsigned prev_taken = CLUSTER && rank > 0 ? peer_address(bars + kSlots, rank - 1) : 0u;
+  bool late = false;
   auto pass_on = [&](int c) {
     if (rank > 0 && lane == 0) slot_arrive(prev_taken, c);
     if (has_next && lane < min(kStep, nd - c * kStep)) {
-      const bool late = c >= kSlots - 1 && slot_wait(bars + kSlots, c - (kSlots - 1), false);
+      if (c >= kSlots - 1) late = slot_wait(bars + kSlots, c - (kSlots - 1), late, tries);
       peer_send(next + 4 * ((c * kStep + lane) & (kEdgeRing - 1)), late ? NAN : own[(c & 1) * kStep + lane],
                 next_full + 8 * (c % kSlots));
     }
@@ -310,8 +319,9 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
       if (keep && c >= 1) weights(c - 1);
     } else if (warp == 0) {
       if (CLUSTER && rank > 0) {
-        if (lane == 0) slot_expect(bars, c, min(kStep, nd - c * kStep));
-        failed = slot_wait(bars, c, failed);
+        // (after a failure no more arrivals: the barrier's phase may not have ended)
+        if (lane == 0 && !failed) slot_expect(bars, c, min(kStep, nd - c * kStep));
+        failed = slot_wait(bars, c, failed, tries);
       }
       float *rw = ringw + (c & 1) * kStep * PITCH + lane * R;
       const float *rx = ringx + (c & 1) * kStep * PITCH + lane * R;
@@ -324,6 +334,7 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
           load_rows<R>(x[s][u], rx + (j0 + u) * PITCH);
           load_rows<R>(y[s][u], ry + (j0 + u) * PITCH);
           nb[s][u] = above[(c * kStep + j0 + u - 1 + off) & (kEdgeRing - 1)];
+          if (CLUSTER && failed) nb[s][u] = NAN;
         }
       };
       auto step = [&](int j, const float (&xs)[R], const float (&ys)[R], float from_above) {
@@ -388,9 +399,9 @@ mi_forward_f32_kernel(const float *__restrict__ px, const float *__restrict__ py
   if (warp == 0) {
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (row0 + i0 + r == box.sb) ans[b] = failed ? NAN : p_cur[r];
+      if (row0 + i0 + r == box.sb) ans[b] = p_cur[r];
   }
-  if (CLUSTER) cluster_sync();  // the neighbours may still be writing here
+  if (CLUSTER) leave_cluster(failed);
 }
 
 // -----------------------------------------------------------------------------
@@ -401,7 +412,7 @@ __global__ void __launch_bounds__(kThreads)
 mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ boundary,
                        const float *__restrict__ ans_grad, float *__restrict__ px_grad,
                        float *__restrict__ py_grad, float *__restrict__ origin_grad, int B, int S, int T,
-                       int row0_arg) {
+                       int row0_arg, int tries) {
   using M = MiShape<R>;
   constexpr int ROWS = M::kRows, PITCH = M::kRing, G = M::kGroup;
   constexpr int off = MODIFIED ? -1 : 0;
@@ -554,11 +565,12 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
   const unsigned previous = CLUSTER && rank > 0 ? peer_address(below, rank - 1) : 0u;
   const unsigned previous_full = CLUSTER && rank > 0 ? peer_address(bars, rank - 1) : 0u;
   const unsigned next_taken = has_next ? peer_address(bars + kSlots, rank + 1) : 0u;
+  bool late = false;
   auto pass_on = [&](int it) {
     const int c = chunk_of(it);
     if (has_next && lane == 0) slot_arrive(next_taken, it);
     if (rank > 0 && lane < min(kStep, nd - c * kStep)) {
-      const bool late = it >= kSlots - 1 && slot_wait(bars + kSlots, it - (kSlots - 1), false);
+      if (it >= kSlots - 1) late = slot_wait(bars + kSlots, it - (kSlots - 1), late, tries);
       peer_send(previous + 4 * ((c * kStep + lane) & (kEdgeRing - 1)), late ? NAN : own[(it & 1) * kStep + lane],
                 previous_full + 8 * (it % kSlots));
     }
@@ -573,8 +585,8 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
       if (it >= 1) drain(it - 1);
     } else if (warp == 0) {
       if (has_next) {
-        if (lane == 0) slot_expect(bars, it, min(kStep, nd - c * kStep));
-        failed = slot_wait(bars, it, failed);
+        if (lane == 0 && !failed) slot_expect(bars, it, min(kStep, nd - c * kStep));
+        failed = slot_wait(bars, it, failed, tries);
       }
       float *rx = ringx + (it & 1) * kStep * PITCH + lane * R;
       float *ry = ringy + (it & 1) * kStep * PITCH + lane * R;
@@ -586,6 +598,7 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
         for (int u = 0; u < G; ++u) {
           load_rows<R>(w[s][u], rw + (j0 + u) * PITCH);
           nb[s][u] = below[(c * kStep + j0 + u + 1 - off) & (kEdgeRing - 1)];
+          if (CLUSTER && failed) nb[s][u] = NAN;
         }
       };
       auto step = [&](int j, const float (&wt)[R], float edge_below) {
@@ -635,16 +648,8 @@ mi_backward_f32_kernel(float *__restrict__ lattice, const int64_t *__restrict__ 
   }
   if (helper && works) drain(nchunks - 1);
   if (sender && works) pass_on(nchunks - 1);
-  if (threadIdx.x == 0 && rank == 0 && row0 == 0 && origin_grad != nullptr) origin_grad[b] = failed ? NAN : g_first;
-  // a wait that ran out: say so where the caller looks (an in-box entry of this CTA's rows)
-  __syncthreads();
-  if (CLUSTER && failed && threadIdx.x == 0) {
-    if (box.tb >= 1)
-      GY[(size_t)(box.s0 + row0 + first) * T + box.t0] = NAN;
-    else if (row0 + first < box.sb)
-      GX[(size_t)(box.s0 + row0 + first) * T1 + box.t0] = NAN;
-  }
-  if (CLUSTER) cluster_sync();  // the neighbours may still be writing here
+  if (threadIdx.x == 0 && rank == 0 && row0 == 0 && origin_grad != nullptr) origin_grad[b] = g_first;
+  if (CLUSTER) leave_cluster(failed);
 }
 
 // -----------------------------------------------------------------------------
@@ -670,21 +675,21 @@ static int launch(Kernel kern, int B, int ranks, size_t smem, cudaStream_t st, A
 
 template <bool MODIFIED, bool WRITE_P>
 static int forward_f32(const float *px, const float *py, const int64_t *boundary, float *p, float *ans,
-                       float *lattice, int B, int S, int T, cudaStream_t st) {
+                       float *lattice, int B, int S, int T, int tries, cudaStream_t st) {
   if (S + 1 <= MiShape<1>::kRows)
     return launch<false>(mi_forward_f32_kernel<1, false, MODIFIED, WRITE_P, false>, B, 1, MiShape<1>::kSmem, st, px,
-                         py, boundary, p, ans, lattice, B, S, T, 0);
+                         py, boundary, p, ans, lattice, B, S, T, 0, tries);
   if (S + 1 <= MiShape<2>::kRows)
     return launch<false>(mi_forward_f32_kernel<2, false, MODIFIED, WRITE_P, false>, B, 1, MiShape<2>::kSmem, st, px,
-                         py, boundary, p, ans, lattice, B, S, T, 0);
+                         py, boundary, p, ans, lattice, B, S, T, 0, tries);
   if (S + 1 <= kMiF32Rows)
     return launch<true>(mi_forward_f32_kernel<2, true, MODIFIED, WRITE_P, false>, B,
                         (S + MiShape<2>::kRows) / MiShape<2>::kRows, MiShape<2>::kSmem, st, px, py, boundary, p, ans,
-                        lattice, B, S, T, 0);
+                        lattice, B, S, T, 0, tries);
   // more rows than one cluster holds: one launch per block of rows, top to bottom
   for (int row0 = 0; row0 <= S; row0 += kMiF32Rows) {
     const int rc = launch<true>(mi_forward_f32_kernel<2, true, MODIFIED, WRITE_P, true>, B, kMaxCluster,
-                                MiShape<2>::kSmem, st, px, py, boundary, p, ans, lattice, B, S, T, row0);
+                                MiShape<2>::kSmem, st, px, py, boundary, p, ans, lattice, B, S, T, row0, tries);
     if (rc != FRNNT_OK) return rc;
   }
   return FRNNT_OK;
@@ -692,21 +697,22 @@ static int forward_f32(const float *px, const float *py, const int64_t *boundary
 
 template <bool MODIFIED>
 static int backward_f32(float *lattice, const int64_t *boundary, const float *ans_grad, float *px_grad,
-                        float *py_grad, float *origin_grad, int B, int S, int T, cudaStream_t st) {
+                        float *py_grad, float *origin_grad, int B, int S, int T, int tries,
+                        cudaStream_t st) {
   if (S + 1 <= MiShape<1>::kRows)
     return launch<false>(mi_backward_f32_kernel<1, false, MODIFIED, false>, B, 1, MiShape<1>::kSmem, st, lattice,
-                         boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, 0);
+                         boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, 0, tries);
   if (S + 1 <= MiShape<2>::kRows)
     return launch<false>(mi_backward_f32_kernel<2, false, MODIFIED, false>, B, 1, MiShape<2>::kSmem, st, lattice,
-                         boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, 0);
+                         boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, 0, tries);
   if (S + 1 <= kMiF32Rows)
     return launch<true>(mi_backward_f32_kernel<2, true, MODIFIED, false>, B,
                         (S + MiShape<2>::kRows) / MiShape<2>::kRows, MiShape<2>::kSmem, st, lattice, boundary,
-                        ans_grad, px_grad, py_grad, origin_grad, B, S, T, 0);
+                        ans_grad, px_grad, py_grad, origin_grad, B, S, T, 0, tries);
   // bottom to top
   for (int row0 = (S / kMiF32Rows) * kMiF32Rows; row0 >= 0; row0 -= kMiF32Rows) {
     const int rc = launch<true>(mi_backward_f32_kernel<2, true, MODIFIED, true>, B, kMaxCluster, MiShape<2>::kSmem,
-                                st, lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, row0);
+                                st, lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, row0, tries);
     if (rc != FRNNT_OK) return rc;
   }
   return FRNNT_OK;
@@ -714,19 +720,20 @@ static int backward_f32(float *lattice, const int64_t *boundary, const float *an
 static_assert(kMaxCluster * MiShape<2>::kRows == kMiF32Rows, "a full cluster holds a block");
 
 int launch_mi_forward_f32(const float *px, const float *py, const int64_t *boundary, float *p, float *ans,
-                          float *lattice, int B, int S, int T, int modified, cudaStream_t st) {
+                          float *lattice, int B, int S, int T, int modified, cudaStream_t st,
+                          int tries) {
   if (p != nullptr)
-    return modified ? forward_f32<true, true>(px, py, boundary, p, ans, lattice, B, S, T, st)
-                    : forward_f32<false, true>(px, py, boundary, p, ans, lattice, B, S, T, st);
-  return modified ? forward_f32<true, false>(px, py, boundary, p, ans, lattice, B, S, T, st)
-                  : forward_f32<false, false>(px, py, boundary, p, ans, lattice, B, S, T, st);
+    return modified ? forward_f32<true, true>(px, py, boundary, p, ans, lattice, B, S, T, tries, st)
+                    : forward_f32<false, true>(px, py, boundary, p, ans, lattice, B, S, T, tries, st);
+  return modified ? forward_f32<true, false>(px, py, boundary, p, ans, lattice, B, S, T, tries, st)
+                  : forward_f32<false, false>(px, py, boundary, p, ans, lattice, B, S, T, tries, st);
 }
 
 int launch_mi_backward_f32(float *lattice, const int64_t *boundary, const float *ans_grad, float *px_grad,
                            float *py_grad, float *origin_grad, int B, int S, int T, int modified,
-                           cudaStream_t st) {
-  return modified ? backward_f32<true>(lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, st)
-                  : backward_f32<false>(lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, st);
+                           cudaStream_t st, int tries) {
+  return modified ? backward_f32<true>(lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, tries, st)
+                  : backward_f32<false>(lattice, boundary, ans_grad, px_grad, py_grad, origin_grad, B, S, T, tries, st);
 }
 
 }  // namespace frnnt

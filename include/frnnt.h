@@ -133,6 +133,16 @@ int frnnt_mi_backward(int dtype, const void *px, const void *py, const int64_t *
                       void *origin_grad, void *lattice, int B, int S, int T, int modified,
                       void *stream);
 
+/* Both float32 sweeps with the waits between the CTAs of a cluster bounded by so many looks at the
+ * barrier (negative: the usual bound; 0: every wait runs out at once), to see what a caller
+ * gets when one does: NaN in every score, lattice value p and gradient that depends on what did
+ * not arrive, in origin_grad too, and no error, since nothing synchronises.  Lattices of up
+ * to 64 rows need no waits.  p and origin_grad may be NULL; `lattice` is 16-byte aligned. */
+int frnnt_mi_sweeps_limited(const float *px, const float *py, const int64_t *boundary,
+                            const float *ans_grad, float *p, float *ans, float *px_grad,
+                            float *py_grad, float *origin_grad, void *lattice, int B, int S, int T,
+                            int modified, int forward_tries, int backward_tries, void *stream);
+
 /* Size of the scratch region built into the library for frnnt_mi_fwd_bwd_noalloc. */
 #define FRNNT_MI_NOALLOC_SCRATCH_BYTES (32u << 20)
 

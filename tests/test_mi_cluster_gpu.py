@@ -80,3 +80,47 @@ def test_scratch_off_a_16_byte_boundary(S, T):
     for a, b in zip(mi.mi_backward_from_lattice(px, lattice, None, w, py.shape),
                     mi.mi_backward_from_lattice(px, moved, None, w, py.shape)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("modified", [False, True])
+@pytest.mark.parametrize("S,T", [(40, 60), (64, 70), (100, 120), (300, 330), (600, 640)])
+def test_a_wait_that_runs_out_shows(S, T, modified):
+    """With no patience at all for the row of the CTA above (below), whatever depends on it is NaN:
+    the lattice from row 64 on and the score, resp. the gradients of the rows above the last CTA's and
+    what reaches the origin.  Nothing hangs, and the next call is right."""
+    from fast_rnnt_b200 import _lib
+    from fast_rnnt_b200._lib import ptr
+    torch.manual_seed(S)
+    B = 3
+    px = (torch.rand(B, S, T + (0 if modified else 1)) * -4).cuda()
+    py = (torch.rand(B, S + 1, T) * -4).cuda()
+    w = torch.ones(B).cuda()
+
+    def sweeps(forward_tries, backward_tries):
+        lattice = torch.zeros(_lib.lib().frnnt_mi_lattice_bytes(0, B, S, T), dtype=torch.uint8, device="cuda")
+        p = torch.zeros(B, S + 1, T + 1).cuda()
+        ans, origin = torch.zeros(B).cuda(), torch.zeros(B).cuda()
+        gx, gy = torch.zeros_like(px), torch.zeros_like(py)
+        _lib.call("frnnt_mi_sweeps_limited", ptr(px), ptr(py), None, ptr(w), ptr(p), ptr(ans), ptr(gx), ptr(gy),
+                  ptr(origin), ptr(lattice), B, S, T, int(modified), forward_tries, backward_tries,
+                  _lib.stream_ptr(px.device))
+        torch.cuda.synchronize()
+        return p, ans, gx, gy, origin
+
+    good = sweeps(-1, -1)
+    reachable = torch.isfinite(good[0])
+    assert reachable[:, S, T].all()
+    p, ans, _, _, _ = sweeps(0, -1)
+    _, _, gx, gy, origin = sweeps(-1, 0)
+    if S + 1 <= 64:   # one CTA
+        assert torch.equal(p, good[0]) and torch.equal(gx, good[2]) and torch.equal(gy, good[3])
+    else:
+        assert torch.equal(p[:, :64], good[0][:, :64])
+        assert torch.isnan(p[:, 64:][reachable[:, 64:]]).all() and torch.isnan(ans).all()
+        last = S // 64 * 64   # first row of the CTA that waits for nobody
+        assert torch.equal(gy[:, last:], good[3][:, last:])
+        # (modified: a cell too late to reach that row depends on nothing there; its gradient is 0)
+        assert torch.isnan(gy[:, :last][good[3][:, :last] != 0]).all() and torch.isnan(origin).all()
+        assert torch.isnan(gx[:, :last - 1][good[2][:, :last - 1] != 0]).all()
+    for a, b in zip(sweeps(-1, -1), good):
+        assert torch.equal(a, b)
