@@ -124,3 +124,21 @@ def test_a_wait_that_runs_out_shows(S, T, modified):
         assert torch.isnan(gx[:, :last - 1][good[2][:, :last - 1] != 0]).all()
     for a, b in zip(sweeps(-1, -1), good):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("modified", [False, True])
+@pytest.mark.parametrize("S,T", [(31, 60), (63, 70), (100, 130), (200, 210), (511, 530), (600, 620)])
+def test_bit_for_bit_as_the_row_per_thread_sweeps(monkeypatch, S, T, modified):
+    """expf and log1pf in the same order: prune ranges, an argmax, move with the last bit."""
+    torch.manual_seed(S)
+    rng = random.Random(S)
+    B = 4
+    px = torch.rand(B, S, T + (0 if modified else 1)) * -4
+    py = torch.rand(B, S + 1, T) * -4
+    for bnd in (None, workloads.random_mi_boundary(B, S, T, modified, rng)):
+        got = run(px, py, bnd, torch.linspace(0.5, 1.5, B))
+        monkeypatch.setenv("FRNNT_MI", "row_per_thread")
+        ref = run(px, py, bnd, torch.linspace(0.5, 1.5, B))
+        monkeypatch.delenv("FRNNT_MI")
+        for a, b in zip(got, ref):
+            assert torch.equal(a, b)
