@@ -204,9 +204,10 @@ size_t frnnt_simple_scratch_bytes(int dtype, int B, int S, int T, int C);
  * of frnnt_lsm_gather_forward and frnnt_pruned_joiner_logprobs_forward means the same. */
 /* 1 if frnnt_simple_logprobs_forward / _backward accept dtype FRNNT_F16 / FRNNT_BF16 (16-bit lm
  * and am, everything else float32) for these sizes: the float32 tensor-core path must apply
- * (C a multiple of 4, ...) and the am-only branch must be off (not smoothed, or
- * am_only_scale == 0), because only that path reads lm and am in a single kernel.  Otherwise
- * convert the inputs to float32 first (same results). */
+ * (any vocabulary; constrained: S + 1 <= 128; saved and scratch 16-byte aligned) and the am-only
+ * branch must be off (not smoothed, or am_only_scale == 0), because only that path has
+ * kernels that read 16-bit lm and am.  Otherwise convert the inputs to float32 first (same results).
+ * The backward reads lm and am, too. */
 int frnnt_simple_reads_16bit_inputs(int S, int T, int C, int rnnt_type, int smoothed,
                                     double am_only_scale);
 

@@ -2,7 +2,7 @@
 same result (used for comparisons when a kernel is tuned):
   FRNNT_CONTRACTION=tf32 | simt   simple lattices on the 3xTF32 engine / on the FMA pipe
                                   instead of the fp16-pair engine,
-  FRNNT_MI=row_per_thread         the lattice backward with one row per thread for all sizes,
+  FRNNT_MI=row_per_thread         the float lattice sweeps with one row per thread for all sizes,
   FRNNT_PAIR_TILE=128             128 x 128 tiles for every fp16-pair product.
 Each alternative must pass the same checks as the default, so that none of them rots."""
 import pytest
